@@ -175,68 +175,163 @@ constexpr double kPivRel = 1e-11;
 
 // The diagonal block (nb <= 64 columns; a narrower last panel is padded with
 // identity rows and columns, which leave the real entries unchanged) in
-// shared memory, 256 threads, thread (r, g) = (t & 63, t >> 6) owning row r's
-// entries of the columns q = g + 4m.  Cholesky, column c in order (a
-// compact loop: the code stays in the instruction cache, which the fully
-// unrolled register version did not): the pivot's square root (pivot test
-// against d0, the matrix's own diagonal, when given), the column divided by
-// it, l_rc l_qc subtracted from the trailing entries -- three barriers a
-// column.  Then the inverse X = L^-1 in place, last column first: X_jj =
-// 1 / L_jj, X_rj = -(sum_{j<q<=r} X_rq L_qj) / L_jj, the four partial sums
-// of each row added in fixed order.  L goes to A's lower triangle, X's
-// strict lower part transposed into A's strict upper triangle (read by the
-// panel TRSM and the inverse factors).
+// shared memory, 256 threads, as a Cholesky of 16-column sub-panels.  It is a
+// serial chain, one CTA's latency per panel of every front, so the layout is
+// chosen for the chain: one warp holds the sub-panel's 16 columns in
+// registers (a lane two rows), so a column costs a shuffle of the pivot, one
+// rsqrt and a multiply, with no barrier; all eight warps subtract the
+// rank-16 product from the columns to its right (8 x 8 tiles on the FP64
+// tensor cores), two barriers a sub-panel.  Pivot test against d0, the
+// matrix's own diagonal, when given.  Then X = L^-1: the four 16 x 16
+// diagonal inverses by substitution in registers, a half warp each, and the
+// blocks below them by distance d from the diagonal, X_ij = -X_ii sum_k L_ik
+// X_kj, as tensor-core tiles (two barriers per distance).  L stays in the
+// lower triangle, X's strict lower part goes transposed to the strict upper
+// one (read by the panel TRSM and the inverse factors), the block is written
+// back in one coalesced pass.  Column-by-column code with three barriers a
+// column took 92 us a launch on the 8 subdomains of the 16^3 mesh and 87 us
+// on the fronts of the 33^3 direct factor; this one 20 and 23 us.
+struct PotrfSmem {
+  double D[kNB][kNB + 4];    // [column][row]: L at row >= column, X(r, c) at [r][c]
+  double T[3][16][20];       // sum_k L_ik X_kj of the blocks of one distance, [blk][k][n]
+  double rinv[kNB];          // 1 / L_jj
+  double d0[kNB];
+};
+
+__device__ __forceinline__ void dmma_8x8x4(double (&d)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+               : "+d"(d[0]), "+d"(d[1])
+               : "d"(a), "d"(b));
+}
+
 __device__ __forceinline__ void potrf_panel(double* __restrict__ A, int32_t fs, int32_t nb,
                                             const double* __restrict__ d0, int32_t* __restrict__ err,
-                                            double (*D)[kNB + 1]) {
-  static_assert(kNB == 64, "the thread layout covers 64 rows in 4 column groups");
-  __shared__ double part[4][kNB];
-  __shared__ double d0s[kNB];
-  __shared__ double piv;
-  const int t = threadIdx.x, r = t & 63, g = t >> 6;
-  if (d0 && t < nb) d0s[t] = fabs(d0[t]);
-  for (int e = t; e < kNB * kNB; e += 256) {
-    const int c = e >> 6, rr = e & 63;
-    D[rr][c] = (rr < nb && c < nb) ? (rr >= c ? A[rr + static_cast<int64_t>(c) * fs] : 0.0) : (rr == c ? 1.0 : 0.0);
+                                            PotrfSmem& sm) {
+  static_assert(kNB == 64, "the warp layout covers 64 rows, two a lane");
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5, fr = lane >> 2, fk = lane & 3;
+  double (*D)[kNB + 4] = sm.D;
+  if (t < kNB) {
+    sm.rinv[t] = 1.0;
+    sm.d0[t] = d0 && t < nb ? fabs(d0[t]) : 0.0;
+  }
+  {
+    const int rr = t & 63;
+    double v[kNB / 4];
+#pragma unroll
+    for (int i = 0; i < kNB / 4; ++i) {
+      const int c = (t >> 6) + 4 * i;
+      v[i] = (rr < nb && c < nb && rr >= c) ? A[rr + static_cast<int64_t>(c) * fs] : (rr == c ? 1.0 : 0.0);
+    }
+#pragma unroll
+    for (int i = 0; i < kNB / 4; ++i) D[(t >> 6) + 4 * i][rr] = v[i];
+  }
+  __syncthreads();
+  const int np = (nb + 15) / 16;  // sub-panels with real columns; the rest is identity
+#pragma unroll 1
+  for (int p = 0; p < np; ++p) {
+    const int c0 = 16 * p, hi = c0 & 32;  // rows hi + lane (and 32 + lane while the pivots are in the first half)
+    if (w == 0) {
+      double a0[16], a1[16];
+#pragma unroll
+      for (int k = 0; k < 16; ++k) {
+        a0[k] = D[c0 + k][hi + lane];
+        a1[k] = hi ? 0.0 : D[c0 + k][32 + lane];
+      }
+#pragma unroll
+      for (int c = 0; c < 16; ++c) {
+        double v = __shfl_sync(0xffffffffu, a0[c], (c0 + c) & 31);
+        if (c0 + c < nb && (!(v > 0.0) || (d0 && !(v > kPivRel * sm.d0[c0 + c])))) {
+          if (lane == 0) atomicOr(err, kErrPivot);
+          // a unit pivot keeps the rest finite; the factorization is reported as failed
+          if (lane == ((c0 + c) & 31)) a0[c] = 1.0;
+          v = 1.0;
+        }
+        const double ri = rsqrt(v);
+        a0[c] *= ri;
+        a1[c] *= ri;
+        if (lane == 0) sm.rinv[c0 + c] = ri;
+#pragma unroll
+        for (int q = c + 1; q < 16; ++q) {
+          const double m = __shfl_sync(0xffffffffu, a0[c], (c0 + q) & 31);
+          a0[q] -= a0[c] * m;
+          a1[q] -= a1[c] * m;
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 16; ++k) {
+        if (hi + lane >= c0 + k) D[c0 + k][hi + lane] = a0[k];
+        if (!hi) D[c0 + k][32 + lane] = a1[k];
+      }
+    }
+    __syncthreads();
+    // trailing 8 x 8 tiles (i >= j) of the columns right of the sub-panel
+    const int n8 = 2 * (np - p - 1), b8 = c0 / 8 + 2;
+    for (int e = w; e < n8 * (n8 + 1) / 2; e += 8) {
+      int i = 0, base = 0;
+      while (base + i + 1 <= e) base += ++i;
+      const int r0 = 8 * (b8 + i), q0 = 8 * (b8 + e - base);
+      double acc[2] = {0.0, 0.0};
+#pragma unroll
+      for (int kk = 0; kk < 16; kk += 4)
+        dmma_8x8x4(acc, D[c0 + kk + fk][r0 + fr], D[c0 + kk + fk][q0 + fr]);
+#pragma unroll
+      for (int q = 0; q < 2; ++q)
+        if (r0 + fr >= q0 + 2 * fk + q) D[q0 + 2 * fk + q][r0 + fr] -= acc[q];
+    }
+    __syncthreads();
+  }
+  // diagonal inverses: half warp h of warps 0 and 1 takes block 2w + h, its lane j column j
+  if (w < 2 && 16 * (2 * w + (lane >> 4)) < 16 * ((np + 1) & ~1)) {
+    const int b0 = 16 * (2 * w + (lane >> 4)), j = lane & 15;
+    double s[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) s[i] = 0.0;
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      const double ri = sm.rinv[b0 + k];
+      const double x = k == j ? ri : (k > j ? -s[k] * ri : 0.0);
+      if (k > j) D[b0 + k][b0 + j] = x;
+#pragma unroll
+      for (int i = k + 1; i < 16; ++i) s[i] += D[b0 + k][b0 + i] * x;
+    }
   }
   __syncthreads();
 #pragma unroll 1
-  for (int c = 0; c < kNB; ++c) {
-    if (t == 0) {
-      double v = D[c][c];
-      if (c < nb && (!(v > 0.0) || (d0 && !(v > kPivRel * d0s[c])))) { atomicOr(err, kErrPivot); v = 1.0; }
-      v = sqrt(v);
-      D[c][c] = v;
-      piv = v;
+  for (int d = 1; d < np; ++d) {
+    const int nq = 4 * (np - d);  // 8 x 8 tiles of the blocks (j + d, j)
+    for (int e = w; e < nq; e += 8) {
+      const int j = e >> 2, i = j + d, ti = (e >> 1) & 1, tj = e & 1;
+      double acc[2] = {0.0, 0.0};
+      for (int k0 = 16 * j; k0 < 16 * i; k0 += 4) {
+        const int k = k0 + fk, n = 16 * j + 8 * tj + fr;
+        const double x = k > n ? D[k][n] : (k == n ? sm.rinv[k] : 0.0);
+        dmma_8x8x4(acc, D[k][16 * i + 8 * ti + fr], x);
+      }
+#pragma unroll
+      for (int q = 0; q < 2; ++q) sm.T[j][8 * ti + fr][8 * tj + 2 * fk + q] = acc[q];
     }
     __syncthreads();
-    if (g == 0 && r > c) D[r][c] /= piv;
-    __syncthreads();
-    if (r > c) {
-      const double lr = D[r][c];
-      for (int q = c + 1 + ((g - c - 1) & 3); q <= r; q += 4) D[r][q] -= lr * D[q][c];
+    for (int e = w; e < nq; e += 8) {
+      const int j = e >> 2, i = j + d, ti = (e >> 1) & 1, tj = e & 1;
+      double acc[2] = {0.0, 0.0};
+#pragma unroll
+      for (int kk = 0; kk < 16; kk += 4) {
+        const int r = 16 * i + 8 * ti + fr, k = 16 * i + kk + fk;
+        const double x = r > k ? D[r][k] : (r == k ? sm.rinv[k] : 0.0);
+        dmma_8x8x4(acc, x, sm.T[j][kk + fk][8 * tj + fr]);
+      }
+#pragma unroll
+      for (int q = 0; q < 2; ++q) D[16 * i + 8 * ti + fr][16 * j + 8 * tj + 2 * fk + q] = -acc[q];
     }
     __syncthreads();
   }
-  for (int e = t; e < nb * nb; e += 256) {
-    const int c = e / nb, rr = e - c * nb;
-    if (rr >= c) A[rr + static_cast<int64_t>(c) * fs] = D[rr][c];
-  }
-#pragma unroll 1
-  for (int j = kNB - 1; j >= 0; --j) {
-    const double ljj = D[j][j];
-    double p = 0.0;
-    if (r > j)
-      for (int q = j + 1 + ((g - j - 1) & 3); q <= r; q += 4) p += D[r][q] * D[q][j];
-    part[g][r] = p;
-    __syncthreads();
-    if (g == 0 && r > j) D[r][j] = -(part[0][r] + part[1][r] + part[2][r] + part[3][r]) / ljj;
-    if (t == 0) D[j][j] = 1.0 / ljj;
-    __syncthreads();
-  }
-  for (int e = t; e < nb * nb; e += 256) {
-    const int rr = e / nb, c = e - rr * nb;
-    if (c < rr) A[c + static_cast<int64_t>(rr) * fs] = D[rr][c];
+  {
+    const int rr = t & 63;
+#pragma unroll
+    for (int i = 0; i < kNB / 4; ++i) {
+      const int c = (t >> 6) + 4 * i;
+      if (rr < nb && c < nb) A[rr + static_cast<int64_t>(c) * fs] = D[c][rr];
+    }
   }
 }
 
@@ -247,7 +342,7 @@ __global__ void __launch_bounds__(256) k_potrf_diag(FrontsDev F, int32_t f0, int
                                                     const double* __restrict__ diag0,
                                                     const int64_t* __restrict__ loc_off, int32_t n_plan,
                                                     int32_t* __restrict__ err) {
-  __shared__ double D[kNB][kNB + 1];
+  __shared__ PotrfSmem sm;
   const int32_t k = f0 + blockIdx.x;
   const int32_t np = F.npiv[k];
   if (k0 >= np) return;
@@ -255,7 +350,7 @@ __global__ void __launch_bounds__(256) k_potrf_diag(FrontsDev F, int32_t f0, int
   const int64_t u0 = rel ? loc_off[F.sub[k]] + F.p0[k] + k0 : 0;
   const int32_t nb = min(kNB, np - k0), fs = F.f[k];
   double* A = fac + F.fac[k] + k0 + static_cast<int64_t>(k0) * fs;
-  potrf_panel(A, fs, nb, rel ? diag0 + u0 : nullptr, err, D);
+  potrf_panel(A, fs, nb, rel ? diag0 + u0 : nullptr, err, sm);
 }
 
 // Asynchronous 8-byte global -> shared copy; `valid` false fills a zero
@@ -354,12 +449,6 @@ struct TileSmemMma {
   double a[2][kGK][kMmaPad];
   double b[2][kGK][kMmaPad];
 };
-
-__device__ __forceinline__ void dmma_8x8x4(double (&d)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
-               : "+d"(d[0]), "+d"(d[1])
-               : "d"(a), "d"(b));
-}
 
 template <bool kOverwrite = false>
 __device__ __forceinline__ void tile_update_mma(double* __restrict__ C, int64_t ldc, int mr, int mc,
