@@ -45,7 +45,7 @@ constexpr int kTile = 64;     // output tile of the rank-k updates
 [[maybe_unused]] constexpr int kKC = 32;  // k-chunk of the FMA (non-tensor-core) rank-k updates
 constexpr double kMinInnerTol = 1e-12;  // floor of a pass's multiplier tolerance
 
-enum : int32_t { kErrPivot = 1, kErrAsm = 2, kErrTc = 4 };
+enum : int32_t { kErrPivot = 1, kErrAsm = 2, kErrTc = 4, kErrWait = 8 };
 
 #define EMG_CK_VOID(call)                                                         \
   do {                                                                            \
@@ -1108,6 +1108,230 @@ __global__ void __launch_bounds__(kPivMax) k_front_bwd_piv(FrontsDev F, int32_t 
   }
 }
 
+// Single-column solves of the levels of larger fronts: one CTA per 64-row
+// block of a front (forward: pivot blocks and update rows alike) or per
+// 64-pivot block (backward), all blocks of all the level's fronts in one
+// launch.  A pivot block I adds up L_IJ y_J over the blocks J before it as
+// they are published (the front's progress counter: blocks finish in order),
+// applies the inverse of its diagonal block, which k_potrf_diag left above
+// the diagonal, publishes its 64 values and moves the counter on; the next
+// tile's entries of L are in flight while it waits.  So the chain of a front
+// costs one hop between CTAs (the counter, 64 values, a 64 x 64 product) per
+// 64 pivots, and the reading of L is spread over as many SMs as the front has
+// blocks.  Blocks are handed out by a ticket, block-major over the fronts:
+// whatever a block waits for has a lower ticket, so it is running or done.
+// Every wait is bounded; one that runs out raises the error word and poisons
+// the block's values, so the solve ends with an error.  With one CTA walking a
+// front's pivot block and a second launch for its update rows a right-hand
+// side took 14.1 ms on the 24^3 direct factor (two passes over the fronts);
+// one pass takes 7.0 ms there and 1.1 ms here.
+constexpr int kRB = kNB;  // rows of a block
+constexpr int kWaitPolls = 1 << 22;
+
+__device__ __forceinline__ int32_t ld_acquire(const int32_t* p) {
+  int32_t v;
+  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_release(int32_t* p, int32_t v) {
+  asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+// Waits until *p >= want; the last value seen, or -1 when the wait ran out.
+__device__ __forceinline__ int32_t wait_progress(const int32_t* p, int32_t want) {
+  for (int i = 0; i < kWaitPolls; ++i) {
+    const int32_t v = ld_acquire(p);
+    if (v >= want) return v;
+  }
+  return -1;
+}
+
+__global__ void __launch_bounds__(256) k_front_fwd_rows(FrontsDev F, int32_t f0, int32_t nf, RhsDev R,
+                                                        const double* __restrict__ fac, int32_t* __restrict__ ticket,
+                                                        int32_t* __restrict__ prog, int32_t* __restrict__ err) {
+  __shared__ int32_t tk;
+  __shared__ double xs[kRB], vs[kRB], ys[2][kRB], part[4][kRB];
+  __shared__ double X[kRB][kRB + 1];  // X[r][c] = (L_II^-1)(r, c)
+  const int t = threadIdx.x, r = t & (kRB - 1), g = t >> 6;
+  if (t == 0) tk = atomicAdd(ticket, 1);
+  __syncthreads();
+  const int32_t b = tk / nf, k = f0 + (tk - b * nf);
+  const int32_t np = F.npiv[k], fs = F.f[k], nu = fs - np, p0 = F.p0[k];
+  const int32_t nbp = (np + kRB - 1) / kRB, nbu = (nu + kRB - 1) / kRB;
+  if (F.is_root[k] || b >= nbp + nbu) return;
+  const bool piv = b < nbp;
+  const int32_t r0 = piv ? b * kRB : np + (b - nbp) * kRB;
+  const int32_t h = min(kRB, (piv ? np : fs) - r0);
+  const int32_t nt = piv ? b : nbp;
+  double* x = R.x + R.off[F.sub[k]] + p0;
+  double* V = R.v + R.voff[k];
+  const double* L = fac + F.fac[k];
+  const double* Lr = L + r0 + r;
+  const bool live = r < h;
+  double ln[16], lc[16];
+  auto fetch = [&](int32_t J) {
+    const int32_t c0 = J * kRB + 16 * g;
+#pragma unroll
+    for (int c = 0; c < 16; ++c) ln[c] = live && c0 + c < np ? __ldcs(Lr + static_cast<int64_t>(c0 + c) * fs) : 0.0;
+  };
+  if (nt > 0) fetch(0);
+  if (t < kRB) xs[t] = piv && t < h ? x[r0 + t] : 0.0;
+  if (piv)
+    for (int e = t; e < kRB * kRB; e += 256) {  // X(r, c), c < r, lies at row c of column r
+      const int c = e & (kRB - 1), rr = e >> 6;
+      double v = 0.0;
+      if (rr < h && c <= rr) {
+        v = L[(r0 + c) + static_cast<int64_t>(r0 + rr) * fs];
+        if (c == rr) v = 1.0 / v;
+      }
+      X[rr][c] = v;
+    }
+  __syncthreads();
+  for (int32_t ci = 0; ci < F.nchild[k]; ++ci) {
+    const int32_t ch = F.child_v[F.child0[k] + ci];
+    const int32_t ncu = F.f[ch] - F.npiv[ch];
+    const double* Vc = R.v + R.voff[ch];
+    const int32_t* cp = F.cpos_v + F.cpos[ch];
+    for (int32_t a = t; a < ncu; a += 256) {
+      const int32_t q = cp[a] - r0;
+      if (q >= 0 && q < h) xs[q] += Vc[a];
+    }
+    __syncthreads();
+  }
+  double acc = 0.0;
+  int32_t seen = 0;
+  for (int32_t J = 0; J < nt; ++J) {
+#pragma unroll
+    for (int c = 0; c < 16; ++c) lc[c] = ln[c];
+    if (J + 1 < nt) fetch(J + 1);
+    if (t < kRB) {
+      if (seen <= J) seen = wait_progress(prog + k, J + 1);
+      if (seen < 0) {
+        if (t == 0) atomicOr(err, kErrWait);
+        seen = INT32_MAX;
+        acc = nan("");
+      }
+      ys[J & 1][t] = J * kRB + t < np ? __ldcg(x + J * kRB + t) : 0.0;
+    }
+    __syncthreads();
+    const double* y = ys[J & 1] + 16 * g;
+#pragma unroll
+    for (int c = 0; c < 16; ++c) acc = fma(lc[c], y[c], acc);
+  }
+  part[g][r] = acc;
+  __syncthreads();
+  if (t < kRB) {
+    const double v = xs[t] - ((part[0][t] + part[1][t]) + (part[2][t] + part[3][t]));
+    if (!piv && t < h) V[r0 - np + t] = v;
+    vs[t] = v;
+  }
+  if (!piv) return;
+  __syncthreads();
+  double s = 0.0;
+#pragma unroll
+  for (int c = 0; c < 16; ++c) s = fma(X[r][16 * g + c], vs[16 * g + c], s);
+  part[g][r] = s;
+  __syncthreads();
+  if (t < h) {
+    x[r0 + t] = (part[0][t] + part[1][t]) + (part[2][t] + part[3][t]);
+    __threadfence();
+  }
+  __syncthreads();
+  if (t == 0) st_release(prog + k, b + 1);
+}
+
+__global__ void __launch_bounds__(256) k_front_bwd_rows(FrontsDev F, int32_t f0, int32_t nf, RhsDev R,
+                                                        const double* __restrict__ fac, int32_t* __restrict__ ticket,
+                                                        int32_t* __restrict__ prog, int32_t* __restrict__ err) {
+  __shared__ int32_t tk;
+  __shared__ double dots[kRB], vs[kRB], part[4][kRB];
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5, r = t & (kRB - 1), g = t >> 6;
+  if (t == 0) tk = atomicAdd(ticket, 1);
+  __syncthreads();
+  const int32_t q = tk / nf, k = f0 + (tk - q * nf);
+  const int32_t np = F.npiv[k], fs = F.f[k];
+  const int32_t nbp = (np + kRB - 1) / kRB, J = nbp - 1 - q;
+  if (F.is_root[k] || J < 0) return;
+  const int32_t c0 = J * kRB, h = min(kRB, np - c0);
+  double* xsub = R.x + R.off[F.sub[k]];
+  double* x = xsub + F.p0[k];
+  const int32_t* rows = F.rows_v + F.rows[k];
+  const double* L = fac + F.fac[k];
+  const double* Lw = L + static_cast<int64_t>(c0 + 8 * w) * fs;  // this warp's 8 columns
+  const int nc = min(8, h - 8 * w);
+  double xr[16];  // X(i, r) for i in 16 g ..: row r of the columns i, coalesced over r
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const int ii = 16 * g + i;
+    double v = 0.0;
+    if (ii < h && r <= ii) {
+      v = L[(c0 + r) + static_cast<int64_t>(c0 + ii) * fs];
+      if (ii == r) v = 1.0 / v;
+    }
+    xr[i] = v;
+  }
+  const double xj = t < h ? x[c0 + t] : 0.0;
+  double acc[8];
+#pragma unroll
+  for (int c = 0; c < 8; ++c) acc[c] = 0.0;
+  for (int32_t i = np + lane; i < fs; i += 64) {  // the update rows: solved by the levels above
+    const bool two = i + 32 < fs;
+    double l0[8], l1[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      l0[c] = c < nc ? __ldcs(Lw + static_cast<int64_t>(c) * fs + i) : 0.0;
+      l1[c] = c < nc && two ? __ldcs(Lw + static_cast<int64_t>(c) * fs + i + 32) : 0.0;
+    }
+    const double x0 = xsub[rows[i]], x1 = two ? xsub[rows[i + 32]] : 0.0;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) acc[c] = fma(l1[c], x1, fma(l0[c], x0, acc[c]));
+  }
+  int32_t seen = 0;
+  double n0[8], n1[8];
+  auto fetch = [&](int32_t I) {
+    const int32_t i0 = I * kRB + lane, i1 = i0 + 32;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      n0[c] = c < nc && i0 < np ? __ldcs(Lw + static_cast<int64_t>(c) * fs + i0) : 0.0;
+      n1[c] = c < nc && i1 < np ? __ldcs(Lw + static_cast<int64_t>(c) * fs + i1) : 0.0;
+    }
+  };
+  if (nbp - 1 > J) fetch(nbp - 1);
+  for (int32_t I = nbp - 1; I > J; --I) {
+    double l0[8], l1[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) { l0[c] = n0[c]; l1[c] = n1[c]; }
+    if (I - 1 > J) fetch(I - 1);
+    if (seen < nbp - I) seen = wait_progress(prog + k, nbp - I);
+    if (seen < 0) {
+      if (lane == 0) atomicOr(err, kErrWait);
+      seen = INT32_MAX;
+      acc[0] = nan("");
+    }
+    const int32_t i0 = I * kRB + lane, i1 = i0 + 32;
+    const double x0 = i0 < np ? __ldcg(x + i0) : 0.0, x1 = i1 < np ? __ldcg(x + i1) : 0.0;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) acc[c] = fma(l1[c], x1, fma(l0[c], x0, acc[c]));
+  }
+  __syncwarp();
+  const double a = warp_reduce_scatter<8>(acc, lane);
+  if (reduce_scatter_writer<8>(lane)) dots[8 * w + reduce_scatter_index<8>(lane)] = a;
+  __syncthreads();
+  if (t < kRB) vs[t] = t < h ? xj - dots[t] : 0.0;
+  __syncthreads();
+  double s = 0.0;
+#pragma unroll
+  for (int i = 0; i < 16; ++i) s = fma(xr[i], vs[16 * g + i], s);
+  part[g][r] = s;
+  __syncthreads();
+  if (t < h) {
+    x[c0 + t] = (part[0][t] + part[1][t]) + (part[2][t] + part[3][t]);
+    __threadfence();
+  }
+  __syncthreads();
+  if (t == 0) st_release(prog + k, q + 1);
+}
+
 // Levels of medium fronts (at most kMidMaxF rows: the leaves and the levels
 // above them): one CTA per (front, group of kC right-hand-side columns) does
 // the front's whole step with the group's front columns held in shared
@@ -1119,6 +1343,13 @@ __global__ void __launch_bounds__(kPivMax) k_front_bwd_piv(FrontsDev F, int32_t 
 // column group, and the small CTAs keep many fronts in flight where the wide
 // pivot-block CTAs would idle on the panel chain.
 constexpr int kMidMaxF = 1024;
+// A single column takes these kernels only on levels of so many fronts that
+// one CTA a front fills the GPU; with fewer, a block per CTA is faster (a
+// right-hand side on the 24^3 direct factor: 1.10 ms with the line at 800
+// fronts, 1.30 at 100, 1.55 with these kernels on every level of medium
+// fronts; 64 subdomains of the 64^3 mesh, 19,842 fronts: 85.7 ms at 800, 88.4
+// at 6,400, 91.7 with a block per CTA on every level).
+constexpr int kMidMinFronts = 800;
 constexpr int kMidCols = 8;     // columns per CTA of the multi-column variant
 template <int kC>
 size_t mid_smem(int32_t max_f) { return sizeof(double) * (static_cast<size_t>(kC) * max_f + kC * kSB); }
@@ -2277,6 +2508,11 @@ int FetiDP::setup_device() {
   EMG_CK(cudaMalloc(&pe, sizeof(int32_t)));
   dev.push_back(pe);
   err_d = static_cast<int32_t*>(pe);
+  EMG_CK(cudaMemsetAsync(err_d, 0, sizeof(int32_t), st));
+  void* pp = nullptr;
+  EMG_CK(cudaMalloc(&pp, sizeof(int32_t) * (2 * (static_cast<size_t>(F) + P.level_ptr.size()))));
+  dev.push_back(pp);
+  prog_d = static_cast<int32_t*>(pp);
   EMG_CK(cudaStreamSynchronize(st));
   return EMG_SUCCESS;
 }
@@ -2290,6 +2526,10 @@ int FetiDP::check_err(const char* where) {
     set_error(std::string(where) + ": non-positive or vanishing pivot (a subdomain matrix is singular or not "
                                     "positive definite)");
     return EMG_NUMERICAL_ERROR;
+  }
+  if (e & kErrWait) {
+    set_error(std::string(where) + ": a front solve gave up waiting for a block of its front");
+    return EMG_ERR_TIMEOUT;
   }
   if (e & kErrTc) {
     set_error(std::string(where) + ": a tensor-core tile gave up waiting for its MMAs");
@@ -2416,6 +2656,7 @@ int FetiDP::solve_fronts(const RhsDev& R, int32_t ncol) {
     lvl_max_np.assign(nlev, 0);
     lvl_max_nu.assign(nlev, 0);
     lvl_max_f.assign(nlev, 0);
+    lvl_max_blk.assign(nlev, 0);
     for (int32_t h = 0; h < nlev; ++h)
       for (int32_t k = plan.level_ptr[h]; k < plan.level_ptr[h + 1]; ++k) {
         const FetiFront& x = plan.fronts[k];
@@ -2423,16 +2664,17 @@ int FetiDP::solve_fronts(const RhsDev& R, int32_t ncol) {
         lvl_max_np[h] = std::max(lvl_max_np[h], x.npiv);
         lvl_max_nu[h] = std::max(lvl_max_nu[h], x.f - x.npiv);
         lvl_max_f[h] = std::max(lvl_max_f[h], x.f);
+        lvl_max_blk[h] = std::max(lvl_max_blk[h], (x.npiv + kRB - 1) / kRB + (x.f - x.npiv + kRB - 1) / kRB);
       }
   }
   const unsigned nc = static_cast<unsigned>(ncol);
   const unsigned ngroups = static_cast<unsigned>((ncol + kColB - 1) / kColB);
   const unsigned ngroups_mid = static_cast<unsigned>((ncol + kMidCols - 1) / kMidCols);
-  // the autotuner's choices are timed on single-column passes and apply to
-  // them; multi-column solves (the coarse basis inside the factorization)
-  // always take the fused kernels on the medium levels, so a factorization's
-  // results do not depend on when the tuner ran
-  const bool use_mid = ncol > 1 || mid_fronts;
+  const int32_t mid_n = ncol > 1 ? 0 : kMidMinFronts;
+  const int32_t F = static_cast<int32_t>(plan.fronts.size());
+  int32_t* tick = prog_d + 2 * static_cast<int64_t>(F);  // per level, forward then backward
+  if (ncol == 1)
+    EMG_CK(cudaMemsetAsync(prog_d, 0, sizeof(int32_t) * (2 * static_cast<size_t>(F) + 2 * nlev), st));
   if (!capturing && ncol > 1)  // up to 8 x 1024 doubles of front columns a CTA
     EMG_CK(cudaFuncSetAttribute(k_front_fwd_mid<kMidCols, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 static_cast<int>(mid_smem<kMidCols>(kMidMaxF))));
@@ -2442,7 +2684,7 @@ int FetiDP::solve_fronts(const RhsDev& R, int32_t ncol) {
   for (int32_t h = 0; h < nlev; ++h) {
     const int32_t f0 = plan.level_ptr[h], nf = plan.level_ptr[h + 1] - f0;
     if (nf == 0) continue;  // (a front without pivots still gathers its children)
-    if (use_mid && lvl_max_f[h] <= kMidMaxF) {
+    if (lvl_max_f[h] <= kMidMaxF && nf >= mid_n) {
       const int32_t ldx = std::max(lvl_max_f[h], 1);
       if (ncol == 1)
         k_front_fwd_mid<1, 128><<<dim3(1, static_cast<unsigned>(nf)), 128, mid_smem<1>(ldx), st>>>(
@@ -2450,6 +2692,12 @@ int FetiDP::solve_fronts(const RhsDev& R, int32_t ncol) {
       else
         k_front_fwd_mid<kMidCols, 256><<<dim3(ngroups_mid, static_cast<unsigned>(nf)), 256,
                                          mid_smem<kMidCols>(ldx), st>>>(fd, f0, R, d_nI, d_nD, fac_d, ldx);
+      continue;
+    }
+    if (ncol == 1) {
+      if (lvl_max_blk[h] > 0)
+        k_front_fwd_rows<<<static_cast<unsigned>(lvl_max_blk[h]) * static_cast<unsigned>(nf), 256, 0, st>>>(
+            fd, f0, nf, R, fac_d, tick + h, prog_d, err_d);
       continue;
     }
     k_front_fwd_piv<<<dim3(nc, static_cast<unsigned>(nf)), piv_threads, 0, st>>>(fd, f0, R, d_nI, d_nD, fac_d);
@@ -2474,7 +2722,7 @@ int FetiDP::solve_fronts(const RhsDev& R, int32_t ncol) {
   for (int32_t h = nlev - 1; h >= 0; --h) {
     const int32_t f0 = plan.level_ptr[h], nf = plan.level_ptr[h + 1] - f0;
     if (nf == 0 || lvl_max_np[h] == 0) continue;
-    if (use_mid && lvl_max_f[h] <= kMidMaxF) {
+    if (lvl_max_f[h] <= kMidMaxF && nf >= mid_n) {
       const int32_t ldx = std::max(lvl_max_f[h], 1);
       if (ncol == 1)
         k_front_bwd_mid<1, 128><<<dim3(1, static_cast<unsigned>(nf)), 128, mid_smem<1>(ldx), st>>>(
@@ -2482,6 +2730,12 @@ int FetiDP::solve_fronts(const RhsDev& R, int32_t ncol) {
       else
         k_front_bwd_mid<kMidCols, 256><<<dim3(ngroups_mid, static_cast<unsigned>(nf)), 256,
                                          mid_smem<kMidCols>(ldx), st>>>(fd, f0, R, d_nI, d_nD, fac_d, ldx);
+      continue;
+    }
+    if (ncol == 1) {
+      const int32_t nb = (lvl_max_np[h] + kRB - 1) / kRB;
+      k_front_bwd_rows<<<static_cast<unsigned>(nb) * static_cast<unsigned>(nf), 256, 0, st>>>(
+          fd, f0, nf, R, fac_d, tick + nlev + h, prog_d + F, err_d);
       continue;
     }
     if (lvl_max_nu[h] > 0)
@@ -2770,14 +3024,15 @@ int FetiDP::factor_device() {
     rc = trtri(n_roots, max_nD, d_rdim, d_rfac, d_roff, Linv_d);  // L^-1 with L^-T above the diagonal
     if (rc) return rc;
   }
-  // Phi = K_rr^-1 K_rP (columns 0..nP-1) and z = K_rr^-1 f_r (column nP)
-  EMG_CK(cudaMemsetAsync(phi_d, 0, sizeof(double) * std::max<int64_t>(phi_size, 1), st));
-  RhsDev R{phi_d, d_roff_s, d_ncol_s, d_voff_s, vs_d};
-  k_setup_rhs<<<dim3(64, static_cast<unsigned>(S)), 256, 0, st>>>(d_loc_off, d_nI, d_nD, d_nP, rp, cl, vl, un.rhs, R);
-  rc = solve_fronts(R, max_ncol);
-  if (rc) return rc;
   const int64_t nc = P.n_coarse;
-  if (nc > 0) {
+  if (nc > 0) {  // without a coarse problem (the direct solver) nothing reads Phi
+    // Phi = K_rr^-1 K_rP (columns 0..nP-1) and z = K_rr^-1 f_r (column nP)
+    EMG_CK(cudaMemsetAsync(phi_d, 0, sizeof(double) * std::max<int64_t>(phi_size, 1), st));
+    RhsDev R{phi_d, d_roff_s, d_ncol_s, d_voff_s, vs_d};
+    k_setup_rhs<<<dim3(64, static_cast<unsigned>(S)), 256, 0, st>>>(d_loc_off, d_nI, d_nD, d_nP, rp, cl, vl, un.rhs,
+                                                                     R);
+    rc = solve_fronts(R, max_ncol);
+    if (rc) return rc;
     int32_t maxw = 0;
     for (int32_t s = 0; s < S; ++s) maxw = std::max(maxw, P.nP[s] * (P.nP[s] + 1));
     if (maxw > 0)
@@ -2820,20 +3075,24 @@ int FetiDP::factor_device() {
 void FetiDP::tune_solve_kernels() {
   const std::string key = "u" + std::to_string(plan.n_union) + "f" + std::to_string(plan.fronts.size()) + "s" +
                           std::to_string(plan.n_parts);
-  RhsDev R1{xu_d, d_roff1, d_ncol1, d_voff1, v1_d};
-  const int32_t saved_upd = upd_rows;
-  mid_fronts = tune::pick("feti.front_mid_levels", key, {1, 0}, [&](int v, cudaStream_t) {
-    mid_fronts = v != 0;
-    solve_fronts(R1, 1);
-  }, st) != 0;
-  piv_threads = tune::pick("feti.front_pivot_threads", key, {512, 256, 1024}, [&](int v, cudaStream_t) {
-    piv_threads = v;
-    solve_fronts(R1, 1);
-  }, st);
-  upd_rows = tune::pick("feti.front_update_rows", key, {saved_upd, 128, 512}, [&](int v, cudaStream_t) {
-    upd_rows = v;
-    solve_fronts(R1, 1);
-  }, st);
+  // the two-kernel front solves run on multi-column solves only (the coarse
+  // basis): timed on the level of the largest fronts, one column
+  int32_t top = -1;
+  for (size_t h = 0; h < lvl_max_np.size(); ++h)
+    if (lvl_max_np[h] > 0 && lvl_max_nu[h] > 0 && (top < 0 || lvl_max_f[h] > lvl_max_f[top])) top = static_cast<int32_t>(h);
+  if (top >= 0 && n_roots > 0) {
+    RhsDev R1{xu_d, d_roff1, d_ncol1, d_voff1, v1_d};
+    const int32_t f0 = plan.level_ptr[top];
+    const unsigned nf = static_cast<unsigned>(plan.level_ptr[top + 1] - f0);
+    piv_threads = tune::pick("feti.front_pivot_threads", key, {512, 256, 1024}, [&](int v, cudaStream_t) {
+      k_front_fwd_piv<<<dim3(1, nf), v, 0, st>>>(fd, f0, R1, d_nI, d_nD, fac_d);
+    }, st);
+    const int32_t saved_upd = upd_rows;
+    upd_rows = tune::pick("feti.front_update_rows", key, {saved_upd, 128, 512}, [&](int v, cudaStream_t) {
+      k_front_fwd_upd<<<dim3(static_cast<unsigned>((lvl_max_nu[top] + v - 1) / v), nf, 1), v, 0, st>>>(
+          fd, f0, R1, d_nI, d_nD, fac_d);
+    }, st);
+  }
   if (n_roots > 0)
     gemv_warps = tune::pick("feti.dense_column_warps", key, {8, 4, 16}, [&](int v, cudaStream_t) {
       const dim3 gr(static_cast<unsigned>((max_nD + v - 1) / v), static_cast<unsigned>(n_roots));
@@ -3093,6 +3352,11 @@ int FetiDP::recover(const double* fu) {
   const FetiPlan& P = plan;
   const int32_t S = P.n_parts;
   const int64_t ne = P.dual_off[S];
+  if (P.n_lambda == 0 && P.n_coarse == 0) {  // nothing couples the subdomains: xu_d = K^-1 fu is prepare_rhs's own
+    k_global_average<<<blocks_for(P.n_dofs, 256), 256, 0, st>>>(P.n_dofs, d_gptr, d_glist, xu_d, xg_d);
+    EMG_CK(cudaGetLastError());
+    return EMG_SUCCESS;
+  }
   RhsDev R{phi_d, d_roff_s, d_ncol_s, d_voff_s, vs_d};
   if (P.n_coarse > 0) {
     if (ne > 0) k_dual_gather<<<blocks_for(ne, 256), 256, 0, st>>>(ne, d_dual_lam, d_dual_sign, nullptr, lam_d, w_d);
@@ -3294,6 +3558,7 @@ int FetiDP::solve(const emg_krylov_config& cfg, const double* b_d, double* x_d, 
     double rr = 0.0;
     rc = global_residual(bg_d, xacc_d, &rr);
     if (rc) return rc;
+    if (!std::isfinite(rr) && (rc = check_err("FETI-DP solve"))) return rc;  // a front solve's wait ran out
     {  // global_residual synchronized the stream: all four events are complete
       float a = 0.f, b = 0.f, c = 0.f;
       cudaEventElapsedTime(&a, ph0.a, ph0.b);

@@ -77,7 +77,6 @@ struct FetiDP {
   bool tc_factor = false;  // factor contractions on the TF32 tensor cores (EMG_FLAG_FACTOR_TF32)
   // CTA widths of the solve kernels (autotuned after the first factorization)
   int32_t piv_threads = 512, upd_rows = 256, gemv_warps = 8;
-  bool mid_fronts = true;  // fused CTA-per-front solve kernels on the levels of medium fronts
   bool tuned = false;
   int32_t precond = 2;  // 0 none, 1 Dirichlet stiffness-scaled, 2 deluxe-scaled, 3 deluxe with FP32 blocks,
                         // 4 deluxe + learned correction (flexible CG)
@@ -107,6 +106,7 @@ struct FetiDP {
   int64_t coarse_fac = 0;
   // extra fronts after the plan's: [0] the coarse matrix, [1 + f] face f's S_a + S_b
   std::vector<int32_t> xnp;
+  std::vector<int32_t> lvl_max_blk;  // most 64-row blocks of a front (pivot and update rows), per level
   std::vector<int32_t> lvl_max_np, lvl_max_nu, lvl_max_f;  // per level, non-root fronts: largest pivot / update
                                                          // counts and front size
   int32_t max_fdim = 0;
@@ -133,6 +133,8 @@ struct FetiDP {
   float *S32_d = nullptr, *fDa32_d = nullptr, *fDb32_d = nullptr, *fDaT32_d = nullptr, *fDbT32_d = nullptr;
   void* state_d = nullptr;
   int32_t* err_d = nullptr;
+  int32_t* prog_d = nullptr;  // single-column front solves: per front its solved blocks (forward, backward), per
+                              // level the block tickets (forward, backward)
   // device-side multiplier loop: one while-loop graph per preconditioner 0..3
   cudaGraphExec_t lam_exec[4] = {nullptr, nullptr, nullptr, nullptr};
   cudaStream_t cap_st = nullptr;
