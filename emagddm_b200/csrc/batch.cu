@@ -14,8 +14,8 @@
 // block that finishes inside a body is skipped until the next list); the
 // slices of the listed blocks are split into equal contiguous shares, one
 // per warp of a one-wave grid, so the remaining work always spreads over the
-// whole GPU.  Every slice writes its own dot-product partials; a warp per
-// block then adds them in slice order -- results do not depend on the grid
+// whole GPU.  Every slice writes its own dot-product partials; a CTA per
+// block then adds them in a fixed order -- results do not depend on the grid
 // or on which blocks are still iterating.
 #include <cuda_runtime.h>
 
@@ -136,36 +136,38 @@ __device__ __forceinline__ void active_slices(const View& B, Body body) {
   }
 }
 
-// Warp per listed block that is not done: the block's per-slice sums added
-// in slice order (lane-strided, then a fixed butterfly), then fin(block, tot).
+// CTA per listed block that is not done: the block's per-slice sums, thread t
+// taking slices t, t + 256, .. in order, then a fixed block sum, then
+// fin(block, tot) in one thread.  A serial chain between two launches of
+// every iteration, so its length is what counts: a block of 32^3 cells has
+// 5,859 slices, six rounds of loads here; with one warp per block it was 23
+// rounds and 15 us a launch (48 blocks of 8^3 .. 32^3 cells), 5 us now.
 template <int K, bool kAll, class Fin>
 __device__ __forceinline__ void finish_blocks(const View& B, Fin fin) {
-  const int lane = threadIdx.x & 31;
+  __shared__ double red[kBT / 32];
   const int nact = B.ctl[5];
-  const int64_t nw = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
-  for (int64_t j = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5; j < nact; j += nw) {
+  for (int j = blockIdx.x; j < nact; j += gridDim.x) {
     const int inst = B.act_inst[j];
     if (!kAll && B.done[inst]) continue;
     double t[K];
 #pragma unroll
     for (int k = 0; k < K; ++k) t[k] = 0.0;
-    // 8 slices a lane in flight, added in slice order
-    constexpr int kU = 8;
+    constexpr int kU = 4;  // slices a thread in flight
     const int64_t s1 = B.inst_slice[inst + 1];
-    for (int64_t s0 = B.inst_slice[inst] + lane; s0 < s1; s0 += 32 * kU) {
+    for (int64_t s0 = B.inst_slice[inst] + threadIdx.x; s0 < s1; s0 += kBT * kU) {
       double v[kU][K];
 #pragma unroll
       for (int u = 0; u < kU; ++u)
 #pragma unroll
-        for (int k = 0; k < K; ++k) v[u][k] = s0 + 32 * u < s1 ? B.partial[(s0 + 32 * u) * K + k] : 0.0;
+        for (int k = 0; k < K; ++k) v[u][k] = s0 + kBT * u < s1 ? B.partial[(s0 + kBT * u) * K + k] : 0.0;
 #pragma unroll
       for (int u = 0; u < kU; ++u)
 #pragma unroll
         for (int k = 0; k < K; ++k) t[k] += v[u][k];
     }
 #pragma unroll
-    for (int k = 0; k < K; ++k) t[k] = warp_sum(t[k]);
-    if (lane == 0) fin(inst, t);
+    for (int k = 0; k < K; ++k) t[k] = block_sum(t[k], red);
+    if (threadIdx.x == 0) fin(inst, t);
   }
 }
 
@@ -706,10 +708,8 @@ int build_plan(DevCsr& A, const std::vector<int64_t>& blocks, cudaStream_t st, B
   return EMG_SUCCESS;
 }
 
-// Warp per block for the per-block sums.
-int fin_grid(int32_t nb) {
-  return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>((nb + kBT / 32 - 1) / (kBT / 32), 148 * 8)));
-}
+// CTA per block for the per-block sums.
+int fin_grid(int32_t nb) { return std::max(1, std::min<int32_t>(nb, 148 * 8)); }
 
 int capture_batch_loop(BatchPlan& P) {
   cudaGraph_t graph = nullptr;
