@@ -12,7 +12,8 @@
 // permuted numbering (P A P^T, P b): all vector kernels stay contiguous; b is
 // permuted on entry and x on exit.  The CSR handed in stays the exported form.
 //
-// One CG iteration:
+// Matrices of at most a few hundred thousand rows run the whole solve in one
+// persistent kernel (krylov_resident.cuh).  Otherwise one CG iteration:
 //   k_cg_spmv_dot   q = A p and p.q        (last block: alpha / breakdown)
 //   k_cg_update     x += a p, r -= a q, z = D^-1 r, r.z and r.r
 //                   (last block: residual, convergence, divergence, beta)
@@ -104,6 +105,11 @@ struct KrylovWorkspace {
   int fuse_grid = 0;
   size_t fuse_smem = 0;
   int64_t fuse_stash = 0;  // entry pairs of a block kept in shared memory
+  // one persistent kernel for the whole solve (krylov_resident.cuh)
+  int res_grid = 0;            // blocks, 0: not available for this matrix
+  double* zp = nullptr;        // (z, old p) pairs
+  int res_shape = 0;           // index into kResShapes
+  int32_t res_room = 0;        // matrix slots that fit a block's shared memory
 };
 
 namespace {
@@ -1302,6 +1308,14 @@ __global__ void k_loop_control(SolverState* st, cudaGraphConditionalHandle handl
   cudaGraphSetConditional(handle, go ? 1u : 0u);
 }
 
+}  // namespace
+}  // namespace emg
+
+#include "krylov_resident.cuh"
+
+namespace emg {
+namespace {
+
 int num_sms() {
   static int n = 0;
   if (!n) {
@@ -1692,6 +1706,87 @@ void launch_update_dir(KrylovWorkspace& w, int64_t n, cudaStream_t st) {
                      w.fuse_stash);
 }
 
+// The persistent kernels: a block per SM (fewer for small matrices: at least
+// kResMinSlices slices each) of the fewest threads that give every row one,
+// two rows a thread at 1024, when cooperative launches are available: up to
+// 303,104 rows on 148 SMs.  The line is where the loop graph is faster: the
+// 37^3 problem (291,708 rows) takes 27.8 ms here and 38.4 with the graph, and
+// with eight rows a thread of 512 to reach further 40^3 takes 44.5 against
+// 46.2 but 46^3 76.4 against 61.7 (the vectors spill and the matrix is read
+// through L2 at a quarter of the graph kernels' occupancy).
+constexpr int64_t kResMinSlices = 8;
+using ResidentKernel = void (*)(ResidentArgs);
+struct ResidentShape {
+  int threads, rows;
+  ResidentKernel cg, bi;
+};
+const ResidentShape kResShapes[] = {{256, 1, k_cg_resident<256, 1>, k_bi_resident<256, 1>},
+                                    {512, 1, k_cg_resident<512, 1>, k_bi_resident<512, 1>},
+                                    {1024, 1, k_cg_resident<1024, 1>, k_bi_resident<1024, 1>},
+                                    {1024, 2, k_cg_resident<1024, 2>, k_bi_resident<1024, 2>}};
+
+void setup_resident(KrylovWorkspace& w) {
+  w.res_grid = 0;
+  int dev = 0, coop = 0, sms = 0, optin = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) {
+    cudaGetLastError();
+    return;
+  }
+  const int64_t ns = (w.n + kSliceRows - 1) / kSliceRows;
+  const int64_t g = std::min<int64_t>(std::min(sms, kResMaxGrid), (ns + kResMinSlices - 1) / kResMinSlices);
+  if (!coop || g < 1 || 3 * kResVals * g > 4 * w.grid) return;
+  const ResidentShape* shape = nullptr;
+  for (const ResidentShape& h : kResShapes)
+    if (!shape && (ns + g - 1) / g <= h.rows * (h.threads / 32)) shape = &h;
+  if (!shape) return;
+  int room = optin;
+  for (ResidentKernel k : {shape->cg, shape->bi}) {
+    cudaFuncAttributes fa;
+    if (cudaFuncGetAttributes(&fa, k) != cudaSuccess) { cudaGetLastError(); return; }
+    room = std::min(room, optin - static_cast<int>(fa.sharedSizeBytes));
+  }
+  if (room < 12 * 32) return;
+  for (ResidentKernel k : {shape->cg, shape->bi}) {
+    int per = 0;
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, room) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, shape->threads, room) != cudaSuccess || per < 1) {
+      cudaGetLastError();
+      return;
+    }
+  }
+  w.res_shape = static_cast<int>(shape - kResShapes);
+  w.res_room = room / 12 / 32 * 32;
+  w.res_grid = static_cast<int>(g);
+}
+
+// The whole solve as one cooperative launch; false when it cannot be launched.
+bool launch_resident(DevCsr& A, const double* b, double* x, int32_t precond, bool bicg, cudaStream_t st) {
+  KrylovWorkspace& w = *A.ws;
+  const Sell& S = *A.sell;
+  const int64_t avg = S.slots / w.res_grid;  // a block's share varies with its rows' lengths
+  const int32_t stage = static_cast<int32_t>(std::min<int64_t>(w.res_room, (2 * avg + 1024) / 32 * 32));
+  const ResidentArgs args{S, b, x, A.row_ptr, A.col, A.val, precond,
+                          reinterpret_cast<double2*>(w.zp), w.z, w.p, reinterpret_cast<unsigned long long*>(w.partial),
+                          w.state, w.hist, w.hist_cap, stage};
+  if (cudaMemsetAsync(w.partial, 0xff, sizeof(double) * 3 * kResVals * w.res_grid, st) != cudaSuccess) return false;
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3(static_cast<unsigned>(w.res_grid));
+  c.blockDim = dim3(static_cast<unsigned>(kResShapes[w.res_shape].threads));
+  c.dynamicSmemBytes = static_cast<size_t>(stage) * 12;
+  c.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  c.attrs = at;
+  c.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&c, bicg ? kResShapes[w.res_shape].bi : kResShapes[w.res_shape].cg, args);
+  if (e != cudaSuccess) cudaGetLastError();
+  return e == cudaSuccess;
+}
+
 int ensure_ws(DevCsr& A, bool bicg, int32_t max_iter, cudaStream_t st) {
   if (!A.ws) {
     A.ws = new KrylovWorkspace();
@@ -1708,6 +1803,8 @@ int ensure_ws(DevCsr& A, bool bicg, int32_t max_iter, cudaStream_t st) {
     if (int rc = pinned_state_alloc(&w.state_h)) return rc;
     EMG_CK(cudaGetDevice(&w.dev));
     setup_fuse(w);
+    setup_resident(w);
+    if (w.res_grid > 0) EMG_CK(cudaMallocAsync(&w.zp, 2 * vb, st));
     if (int rc = take_stream(&w.cap)) return rc;
     if (int rc = take_event(&w.ev0)) return rc;
     if (int rc = take_event(&w.ev1)) return rc;
@@ -1852,6 +1949,25 @@ int capture_chunk(DevCsr& A, bool bicg, cudaGraphExec_t* out) {
   return EMG_SUCCESS;
 }
 
+// The result of a finished solve from the state read back.
+int finish_solver(KrylovWorkspace& w, bool done, emg_result* res) {
+  float ms = 0.0f;
+  EMG_CK(cudaEventElapsedTime(&ms, w.ev0, w.ev1));
+  if (!done) {
+    set_error("solver state did not finish within the iteration bound");
+    res->status = EMG_ERR_INTERNAL;
+    return EMG_ERR_INTERNAL;
+  }
+  const SolverState& s = *w.state_h;
+  res->status = s.status;
+  res->iterations = s.iter;
+  res->residual_norm = s.res;
+  res->solve_time_ms = ms;
+  w.hist_len = s.iter < w.hist_cap ? s.iter : w.hist_cap;
+  if (w.hist_len < 0) w.hist_len = 0;
+  return s.status;
+}
+
 int run_solver(DevCsr& A, const double* b, double* x, const emg_krylov_config& cfg,
                cudaStream_t user, emg_result* res, bool bicg) {
   std::memset(res, 0, sizeof(*res));
@@ -1875,6 +1991,23 @@ int run_solver(DevCsr& A, const double* b, double* x, const emg_krylov_config& c
   }
   trace_pool("solve.sell.end");
   if (rc) { res->status = rc; return rc; }
+  const Sell& S = *A.sell;
+  SolverState init;
+  std::memset(&init, 0, sizeof(init));
+  init.tol = cfg.tolerance;
+  init.max_iter = max_iter;
+  init.loop_limit = (max_iter > 0 ? max_iter : 0) / kBody + 2;
+  *w.state_h = init;
+  EMG_CK(cudaEventRecord(w.ev0, st));
+  EMG_CK(cudaMemcpyAsync(w.state, w.state_h, sizeof(SolverState), cudaMemcpyHostToDevice, st));
+  const int g = w.grid;
+  bool done = false;
+  if (w.res_grid > 0 && launch_resident(A, b, x, cfg.preconditioner, bicg, st)) {
+    EMG_CK(cudaEventRecord(w.ev1, st));
+    EMG_CK(cudaMemcpyAsync(w.state_h, w.state, sizeof(SolverState), cudaMemcpyDeviceToHost, st));
+    EMG_CK(cudaStreamSynchronize(st));
+    return finish_solver(w, w.state_h->done != 0, res);
+  }
   // Preferred: the whole solve as one graph with a device while-loop; else
   // host-polled chunks of kChunk iterations.
   cudaGraphExec_t* loop = bicg ? &w.bi_loop : &w.cg_loop;
@@ -1901,16 +2034,6 @@ int run_solver(DevCsr& A, const double* b, double* x, const emg_krylov_config& c
     }
     if (rc) { res->status = rc; return rc; }
   }
-  const Sell& S = *A.sell;
-  SolverState init;
-  std::memset(&init, 0, sizeof(init));
-  init.tol = cfg.tolerance;
-  init.max_iter = max_iter;
-  init.loop_limit = (max_iter > 0 ? max_iter : 0) / kBody + 2;
-  *w.state_h = init;
-  EMG_CK(cudaEventRecord(w.ev0, st));
-  EMG_CK(cudaMemcpyAsync(w.state, w.state_h, sizeof(SolverState), cudaMemcpyHostToDevice, st));
-  const int g = w.grid;
   k_jacobi<<<g, kThreads, 0, st>>>(A.n, A.row_ptr, A.col, A.val, S.perm, cfg.preconditioner, w.dinv);
   if (!bicg)
     k_cg_init<<<g, kThreads, 0, st>>>(A.n, b, S.perm, w.dinv, w.x, w.r, w.z, w.p, w.partial, w.state);
@@ -1919,7 +2042,6 @@ int run_solver(DevCsr& A, const double* b, double* x, const emg_krylov_config& c
   EMG_CK(cudaGetLastError());
   // Graph chunks until the device state says done; bounded by max_iter.
   const int64_t max_chunks = (static_cast<int64_t>(max_iter > 0 ? max_iter : 0) + kChunk - 1) / kChunk + 1;
-  bool done = false;
   if (*loop) {
     EMG_CK(cudaGraphLaunch(*loop, st));
     k_scatter<<<g, kThreads, 0, st>>>(A.n, S.perm, w.x, x);
@@ -1938,21 +2060,7 @@ int run_solver(DevCsr& A, const double* b, double* x, const emg_krylov_config& c
     EMG_CK(cudaEventRecord(w.ev1, st));
     EMG_CK(cudaStreamSynchronize(st));
   }
-  float ms = 0.0f;
-  EMG_CK(cudaEventElapsedTime(&ms, w.ev0, w.ev1));
-  if (!done) {
-    set_error("solver state did not finish within the iteration bound");
-    res->status = EMG_ERR_INTERNAL;
-    return EMG_ERR_INTERNAL;
-  }
-  const SolverState& s = *w.state_h;
-  res->status = s.status;
-  res->iterations = s.iter;
-  res->residual_norm = s.res;
-  res->solve_time_ms = ms;
-  w.hist_len = s.iter < w.hist_cap ? s.iter : w.hist_cap;
-  if (w.hist_len < 0) w.hist_len = 0;
-  return s.status;
+  return finish_solver(w, done, res);
 }
 
 }  // namespace
@@ -2073,7 +2181,7 @@ void free_workspace(KrylovWorkspace* w) {
   }
   {
     TraceScope t("free_workspace.vectors");
-    for (double* p : {w->dinv, w->x, w->r, w->z, w->p, w->q, w->rh, w->v, w->s, w->t, w->partial, w->hist})
+    for (double* p : {w->dinv, w->x, w->r, w->z, w->p, w->q, w->rh, w->v, w->s, w->t, w->partial, w->hist, w->zp})
       if (p) cudaFreeAsync(p, 0);
     if (w->state) cudaFreeAsync(w->state, 0);
   }
