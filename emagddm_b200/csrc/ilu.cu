@@ -8,9 +8,10 @@
 // lower) and U (upper with the diagonal) on A's own sparsity pattern, the
 // classic row-by-row (IKJ) elimination restricted to that pattern.  Rows are
 // grouped into levels (a row's level is one more than the highest level of
-// the rows its lower part depends on), so the factorization and the two
-// triangular solves run as one kernel launch per level, warps or 8-lane
-// groups per row; a zero or non-finite pivot counts as a failed
+// the rows its lower part depends on), so the factorization runs as one kernel
+// launch per level, a warp per row, and the two triangular solves level by
+// level in one block (k_ilu_sweeps) or, for levels of many rows, as one launch
+// per level, 8 lanes per row; a zero or non-finite pivot counts as a failed
 // factorization and, as in the reference, the solve then runs without a
 // preconditioner.  Different fill than IncompleteLUT's gives different
 // iteration counts; the converged solution is the same.
@@ -46,6 +47,7 @@ struct IlState {
   double bnorm, rz, rho, alpha, beta, omega, res, prev;
   double tol;
   int32_t iter, max_iter, status, done, early, div_count, loops, loop_limit;
+  uint32_t ticket;  // blocks of the running kernel that have published their partial sums
 };
 
 enum Step : int32_t {
@@ -64,6 +66,94 @@ enum Step : int32_t {
 
 __device__ __forceinline__ int64_t gtid() { return static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; }
 __device__ __forceinline__ int64_t gsize() { return static_cast<int64_t>(gridDim.x) * blockDim.x; }
+
+// One step of the scalar recurrence from the totals s0, s1 (one thread).
+__device__ void il_step(IlState* st, int32_t step, double s0, double s1) {
+  const int32_t it = st->iter;
+  switch (step) {
+    case kInitB: st->bnorm = sqrt(s0); break;
+    case kInitCg: st->rz = s0; break;
+    case kInitBi: st->rho = s0; break;
+    case kCgPq:
+      if (fabs(s0) < 1e-30) { st->status = EMG_NUMERICAL_ERROR; st->done = 1; }
+      else st->alpha = st->rz / s0;
+      break;
+    case kCgRr: st->res = sqrt(s0) / st->bnorm; break;
+    case kCgRz: {
+      const double res = st->res;
+      if (res < st->tol) { st->status = EMG_SUCCESS; st->done = 1; break; }
+      if (it > 10 && res > st->prev * 1000.0) { st->status = EMG_DIVERGED; st->done = 1; break; }
+      st->beta = s0 / st->rz;
+      st->rz = s0;
+      st->prev = res;
+      if (it >= st->max_iter) { st->status = EMG_MAX_ITER_REACHED; st->done = 1; }
+      else st->iter = it + 1;
+      break;
+    }
+    case kBiRho: {
+      const double rho_old = st->rho;
+      st->rho = s0;
+      if (fabs(s0) < 1e-30) { st->status = EMG_NUMERICAL_ERROR; st->done = 1; break; }
+      st->beta = (s0 / rho_old) * (st->alpha / st->omega);
+      break;
+    }
+    case kBiRv:
+      if (fabs(s0) < 1e-30) { st->status = EMG_NUMERICAL_ERROR; st->done = 1; }
+      else st->alpha = st->rho / s0;
+      break;
+    case kBiSs: {
+      const double res = sqrt(s0) / st->bnorm;
+      st->res = res;
+      if (res < st->tol) { st->status = EMG_SUCCESS; st->done = 1; st->early = 1; }
+      break;
+    }
+    case kBiTt: st->omega = fabs(s0) < 1e-30 ? 0.0 : s1 / s0; break;
+    case kBiRr: {
+      const double res = sqrt(s0) / st->bnorm;
+      st->res = res;
+      if (res < st->tol) { st->status = EMG_SUCCESS; st->done = 1; break; }
+      if (res > st->prev * 1.5 && it > 20) {
+        if (++st->div_count >= 3) { st->status = EMG_DIVERGED; st->done = 1; break; }
+      } else {
+        st->div_count = 0;
+      }
+      if (it > 10 && res > st->prev * 1000.0) { st->status = EMG_DIVERGED; st->done = 1; break; }
+      st->prev = res;
+      if (it >= st->max_iter) { st->status = EMG_MAX_ITER_REACHED; st->done = 1; }
+      else st->iter = it + 1;
+      break;
+    }
+    default: break;
+  }
+}
+
+// The block's share of up to two sums; the last block to arrive adds all
+// blocks' shares in block order and takes the step.
+__device__ __forceinline__ void il_finish(double a0, double a1, double* partial, IlState* st, int32_t step) {
+  __shared__ double red[kIlThreads / 32];
+  __shared__ bool last;
+  const double b0 = block_sum(a0, red);
+  const double b1 = block_sum(a1, red);
+  if (threadIdx.x == 0) {
+    partial[blockIdx.x] = b0;
+    partial[gridDim.x + blockIdx.x] = b1;
+    __threadfence();
+    last = atomicAdd(&st->ticket, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  double c0 = 0.0, c1 = 0.0;
+  for (int i = threadIdx.x; i < static_cast<int>(gridDim.x); i += blockDim.x) {
+    c0 += ld_l2(partial + i);
+    c1 += ld_l2(partial + gridDim.x + i);
+  }
+  const double s0 = block_sum(c0, red);
+  const double s1 = block_sum(c1, red);
+  if (threadIdx.x != 0) return;
+  st->ticket = 0;
+  il_step(st, step, s0, s1);
+}
 
 // ----------------------------------------------------------- factorization
 
@@ -147,18 +237,161 @@ __global__ void __launch_bounds__(kIlThreads) k_ilu_upper(const int32_t* __restr
   if (i >= 0 && sub == 0) z[i] = (y[i] - s) / lu[diag[i]];
 }
 
-// ------------------------------------------------------- vector kernels
+// Both triangular solves in one launch of one block, for matrices whose levels
+// are too small to fill more.  The solves are a chain of levels (178 of about
+// 125 rows each for the 16^3 system), so what counts is the step from level
+// to level: with a launch per level 2.8 us, here a block barrier, a gather
+// from shared memory and a row's few multiply-adds, 0.4 us (16^3 solve 140 ->
+// 28 ms).
+//   Rows are stored in level order in chunks of 32 (padded), a lane a row, its
+// entries in groups of four for 16-byte loads; chunk c belongs to warp c mod 16, so that with a few chunks a level a
+// warp has several levels' time between its chunks: right after the barrier
+// that ends its level it loads the next chunk's entries and right-hand side
+// into registers (its offsets and indices came one chunk earlier still), off
+// the path of the warps that work on the level now.  The last kIlRing solved
+// values lie in a ring in shared memory; older ones are read back from global
+// memory (which is which is known when the rows are laid out).
+constexpr int kIlWarps = 16;
+constexpr int kIlRing = 12288;  // values (96 KB; a multiple of 32)
+constexpr int kIlGroups = 2;  // groups of four entries of a row held in registers; the rest are loaded when used
 
-// Per-block partial sums of up to two products, partial[k * gridDim + block].
-__device__ __forceinline__ void write_partials(double a0, double a1, double* partial) {
-  __shared__ double red[kIlThreads / 32];
-  const double b0 = block_sum(a0, red);
-  const double b1 = block_sum(a1, red);
-  if (threadIdx.x == 0) {
-    partial[blockIdx.x] = b0;
-    partial[gridDim.x + blockIdx.x] = b1;
+struct IlSweep {
+  int32_t nlev = 0, nchunk = 0;
+  int64_t groups = 0;       // entry groups of all chunks (32 rows x 4 entries each)
+  int32_t* lev = nullptr;   // nlev + 1: first chunk of every level
+  int32_t* off = nullptr;   // nchunk + 1: first entry group of every chunk
+  int32_t* in = nullptr;    // 32 nchunk: index of the row's right-hand side, -1 = padding
+  int32_t* row = nullptr;   // 32 nchunk: matrix row, -1 = padding
+  int4* pos = nullptr;      // [group][lane]: four entries' columns: the ring slot, or ~position once it has left the ring
+  int32_t* src = nullptr;   // [group][lane][4]: their index in the factor, -1 = padding
+  double2* val = nullptr;   // [group][2][lane]: their values, refreshed with every factorization
+  double* dinv = nullptr;   // 32 nchunk: 1 / u_ii (null: unit diagonal)
+};
+
+__device__ __forceinline__ void il_sweep(const IlSweep& S, const double* in, double* out, double* z, double* ring,
+                                         const int32_t* lev) {
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  constexpr int E = 4 * kIlGroups;
+  int32_t c = w;  // this warp's next chunk; its data below
+  int32_t slot = 32 * w + lane;  // its ring slot: 32 c + lane modulo the ring
+  int32_t pp[E], len = 0, off = 0, row = -1;
+  double pv[E], rhs = 0.0, di = 1.0;
+  int32_t off1 = 0, len1 = 0, idx1 = -1, row1 = -1;  // offsets and indices of the chunk after it
+  auto meta = [&](int32_t k) {
+    idx1 = row1 = -1;
+    len1 = 0;
+    if (k < S.nchunk) {
+      off1 = S.off[k];
+      len1 = S.off[k + 1] - off1;
+      idx1 = S.in[32 * k + lane];
+      if (z) row1 = S.row[32 * k + lane];
+    }
+  };
+  auto load = [&](int32_t g, int32_t* p, double* v) {
+    const int4 a = S.pos[32 * g + lane];
+    const double2 x = S.val[64 * g + lane], y = S.val[64 * g + 32 + lane];
+    p[0] = a.x; p[1] = a.y; p[2] = a.z; p[3] = a.w;
+    v[0] = x.x; v[1] = x.y; v[2] = y.x; v[3] = y.y;
+  };
+  auto fetch = [&](int32_t k) {  // the chunk whose offsets are in off1 / len1 / idx1
+    off = off1;
+    len = len1;
+#pragma unroll
+    for (int g = 0; g < kIlGroups; ++g) {
+      if (g < len) {
+        load(off + g, pp + 4 * g, pv + 4 * g);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) { pp[4 * g + j] = lane; pv[4 * g + j] = 0.0; }
+      }
+    }
+    rhs = idx1 >= 0 ? in[idx1] : 0.0;
+    di = S.dinv && idx1 >= 0 ? S.dinv[32 * k + lane] : 1.0;
+    row = row1;
+    meta(k + kIlWarps);
+  };
+  meta(c);
+  fetch(c);
+  for (int32_t l = 1; l <= S.nlev; ++l) {
+    const int32_t e1 = lev[l];
+    bool pending = false;
+    while (c < e1) {
+      if (pending) fetch(c);
+      double g[E], s = 0.0, s1 = 0.0;
+      bool far = false;
+#pragma unroll
+      for (int j = 0; j < E; ++j) {
+        g[j] = ring[max(pp[j], 0)];
+        far |= pp[j] < 0;
+      }
+      if (__any_sync(0xffffffffu, far)) {
+#pragma unroll
+        for (int j = 0; j < E; ++j)
+          if (pp[j] < 0) g[j] = out[~pp[j]];
+      }
+#pragma unroll
+      for (int j = 0; j < E; j += 2) {
+        s = fma(pv[j], g[j], s);
+        s1 = fma(pv[j + 1], g[j + 1], s1);
+      }
+      for (int q = kIlGroups; q < len; ++q) {
+        int32_t p[4];
+        double v[4];
+        load(off + q, p, v);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) s = fma(v[j], p[j] < 0 ? out[~p[j]] : ring[p[j]], s);
+      }
+      const double v = (rhs - (s + s1)) * di;
+      const int32_t p = 32 * c + lane;
+      ring[slot] = v;
+      out[p] = v;
+      if (row >= 0) z[row] = v;
+      c += kIlWarps;
+      slot += 32 * kIlWarps;
+      if (slot >= kIlRing) slot -= kIlRing;
+      pending = true;
+    }
+    __syncthreads();
+    if (pending) fetch(c);
   }
 }
+
+// The line between one block and a launch per level lies at this many rows a
+// level on average: 507 (32^3) 333 ms a solve against 593, 1,144 (48^3) 1.97 s
+// against 1.86 (the one SM's bandwidth, about 55 GB/s here, is what bounds it).
+constexpr int64_t kIlMaxRows = 1000;
+constexpr int kIlMaxLevels = 8000;  // of a sweep: the level offsets of both lie beside the ring
+size_t ilu_sweep_smem(int32_t nl, int32_t nu) { return sizeof(double) * kIlRing + sizeof(int32_t) * (nl + nu + 2); }
+
+// z = U^-1 L^-1 r
+__global__ void __launch_bounds__(32 * kIlWarps) k_ilu_sweeps(IlSweep L, IlSweep U, const double* r, double* ypos,
+                                                              double* zpos, double* z,
+                                                              const IlState* __restrict__ st) {
+  extern __shared__ __align__(16) double il_ring[];
+  if (st->done) return;
+  int32_t* lev = reinterpret_cast<int32_t*>(il_ring + kIlRing);  // both sweeps' level offsets
+  for (int i = threadIdx.x; i < kIlRing; i += blockDim.x) il_ring[i] = 0.0;
+  for (int i = threadIdx.x; i <= L.nlev; i += blockDim.x) lev[i] = L.lev[i];
+  for (int i = threadIdx.x; i <= U.nlev; i += blockDim.x) lev[L.nlev + 1 + i] = U.lev[i];
+  __syncthreads();
+  il_sweep(L, r, ypos, nullptr, il_ring, lev);
+  il_sweep(U, ypos, zpos, z, il_ring, lev + L.nlev + 1);
+}
+
+// Values of a sweep's entries (and 1 / u_ii) from the factor.
+__global__ void k_ilu_pack(IlSweep S, const double* __restrict__ lu,
+                           const int32_t* __restrict__ diag) {
+  for (int64_t i = gtid(); i < 64 * S.groups; i += gsize()) {  // [group][half][lane]
+    const int64_t g = i >> 6, lane = i & 31, half = (i >> 5) & 1;
+    const int32_t* e = S.src + (32 * g + lane) * 4 + 2 * half;
+    S.val[i] = make_double2(e[0] >= 0 ? lu[e[0]] : 0.0, e[1] >= 0 ? lu[e[1]] : 0.0);
+  }
+  if (S.dinv)
+    for (int64_t i = gtid(); i < 32 * static_cast<int64_t>(S.nchunk); i += gsize())
+      S.dinv[i] = S.row[i] >= 0 ? 1.0 / lu[diag[S.row[i]]] : 1.0;
+}
+
+// ------------------------------------------------------- vector kernels
 
 // y = A x (CSR, kIlLanes lanes a row); partials w0.y (w0 null: y.y) and w1.y.
 __global__ void __launch_bounds__(kIlThreads) k_il_spmv(int64_t n, const int32_t* __restrict__ rp,
@@ -166,7 +399,7 @@ __global__ void __launch_bounds__(kIlThreads) k_il_spmv(int64_t n, const int32_t
                                                         const double* __restrict__ val,
                                                         const double* __restrict__ x, double* __restrict__ y,
                                                         const double* __restrict__ w0, const double* __restrict__ w1,
-                                                        double* partial, const IlState* __restrict__ st) {
+                                                        double* partial, IlState* st, int32_t step) {
   if (st->done) return;
   const int sub = threadIdx.x & (kIlLanes - 1);
   double a0 = 0.0, a1 = 0.0;
@@ -185,23 +418,23 @@ __global__ void __launch_bounds__(kIlThreads) k_il_spmv(int64_t n, const int32_t
       if (w1) a1 += w1[row] * s;
     }
   }
-  write_partials(a0, a1, partial);
+  il_finish(a0, a1, partial, st, step);
 }
 
 // partials of a.b
 __global__ void __launch_bounds__(kIlThreads) k_il_dot(int64_t n, const double* __restrict__ a,
                                                        const double* __restrict__ b, double* partial,
-                                                       const IlState* __restrict__ st) {
+                                                       IlState* st, int32_t step) {
   if (st->done) return;
   double acc = 0.0;
   for (int64_t i = gtid(); i < n; i += gsize()) acc += a[i] * b[i];
-  write_partials(acc, 0.0, partial);
+  il_finish(acc, 0.0, partial, st, step);
 }
 
 // CG: x += alpha p, r -= alpha q; partials r.r
 __global__ void __launch_bounds__(kIlThreads) k_il_cg_xr(int64_t n, double* __restrict__ x, double* __restrict__ r,
                                                          const double* __restrict__ p, const double* __restrict__ q,
-                                                         double* partial, const IlState* __restrict__ st) {
+                                                         double* partial, IlState* st, int32_t step) {
   if (st->done) return;
   const double a = st->alpha;
   double acc = 0.0;
@@ -211,7 +444,7 @@ __global__ void __launch_bounds__(kIlThreads) k_il_cg_xr(int64_t n, double* __re
     r[i] = ri;
     acc += ri * ri;
   }
-  write_partials(acc, 0.0, partial);
+  il_finish(acc, 0.0, partial, st, step);
 }
 
 // CG: p = z + beta p
@@ -233,7 +466,7 @@ __global__ void k_il_bi_p(int64_t n, double* __restrict__ p, const double* __res
 // BiCGSTAB: s = r - alpha v; partials s.s
 __global__ void __launch_bounds__(kIlThreads) k_il_bi_s(int64_t n, double* __restrict__ s,
                                                         const double* __restrict__ r, const double* __restrict__ v,
-                                                        double* partial, const IlState* __restrict__ st) {
+                                                        double* partial, IlState* st, int32_t step) {
   if (st->done) return;
   const double a = st->alpha;
   double acc = 0.0;
@@ -242,7 +475,7 @@ __global__ void __launch_bounds__(kIlThreads) k_il_bi_s(int64_t n, double* __res
     s[i] = si;
     acc += si * si;
   }
-  write_partials(acc, 0.0, partial);
+  il_finish(acc, 0.0, partial, st, step);
 }
 
 // BiCGSTAB early exit on ||s||: x += alpha p (:1174-1182)
@@ -257,7 +490,7 @@ __global__ void k_il_bi_early(int64_t n, double* __restrict__ x, const double* _
 __global__ void __launch_bounds__(kIlThreads) k_il_bi_xr(int64_t n, double* __restrict__ x, double* __restrict__ r,
                                                          const double* __restrict__ p, const double* __restrict__ z,
                                                          const double* __restrict__ s, const double* __restrict__ t,
-                                                         double* partial, const IlState* __restrict__ st) {
+                                                         double* partial, IlState* st, int32_t step) {
   if (st->done) return;
   const double a = st->alpha, w = st->omega;
   double acc = 0.0;
@@ -267,78 +500,7 @@ __global__ void __launch_bounds__(kIlThreads) k_il_bi_xr(int64_t n, double* __re
     r[i] = ri;
     acc += ri * ri;
   }
-  write_partials(acc, 0.0, partial);
-}
-
-// One step of the scalar recurrence from the partials of the last kernel.
-__global__ void __launch_bounds__(kIlThreads) k_il_step(const double* __restrict__ partial, int32_t np, IlState* st,
-                                                        int32_t step) {
-  __shared__ double red[kIlThreads / 32];
-  if (step != kInitB && step != kInitCg && step != kInitBi && st->done) return;
-  double a0 = 0.0, a1 = 0.0;
-  for (int i = threadIdx.x; i < np; i += blockDim.x) {
-    a0 += partial[i];
-    a1 += partial[np + i];
-  }
-  const double s0 = block_sum(a0, red);
-  const double s1 = block_sum(a1, red);
-  if (threadIdx.x != 0) return;
-  const int32_t it = st->iter;
-  switch (step) {
-    case kInitB: st->bnorm = sqrt(s0); break;
-    case kInitCg: st->rz = s0; break;
-    case kInitBi: st->rho = s0; break;
-    case kCgPq:
-      if (fabs(s0) < 1e-30) { st->status = EMG_NUMERICAL_ERROR; st->done = 1; }
-      else st->alpha = st->rz / s0;
-      break;
-    case kCgRr: st->res = sqrt(s0) / st->bnorm; break;
-    case kCgRz: {
-      const double res = st->res;
-      if (res < st->tol) { st->status = EMG_SUCCESS; st->done = 1; break; }
-      if (it > 10 && res > st->prev * 1000.0) { st->status = EMG_DIVERGED; st->done = 1; break; }
-      st->beta = s0 / st->rz;
-      st->rz = s0;
-      st->prev = res;
-      if (it >= st->max_iter) { st->status = EMG_MAX_ITER_REACHED; st->done = 1; }
-      else st->iter = it + 1;
-      break;
-    }
-    case kBiRho: {
-      const double rho_old = st->rho;
-      st->rho = s0;
-      if (fabs(s0) < 1e-30) { st->status = EMG_NUMERICAL_ERROR; st->done = 1; break; }
-      st->beta = (s0 / rho_old) * (st->alpha / st->omega);
-      break;
-    }
-    case kBiRv:
-      if (fabs(s0) < 1e-30) { st->status = EMG_NUMERICAL_ERROR; st->done = 1; }
-      else st->alpha = st->rho / s0;
-      break;
-    case kBiSs: {
-      const double res = sqrt(s0) / st->bnorm;
-      st->res = res;
-      if (res < st->tol) { st->status = EMG_SUCCESS; st->done = 1; st->early = 1; }
-      break;
-    }
-    case kBiTt: st->omega = fabs(s0) < 1e-30 ? 0.0 : s1 / s0; break;
-    case kBiRr: {
-      const double res = sqrt(s0) / st->bnorm;
-      st->res = res;
-      if (res < st->tol) { st->status = EMG_SUCCESS; st->done = 1; break; }
-      if (res > st->prev * 1.5 && it > 20) {
-        if (++st->div_count >= 3) { st->status = EMG_DIVERGED; st->done = 1; break; }
-      } else {
-        st->div_count = 0;
-      }
-      if (it > 10 && res > st->prev * 1000.0) { st->status = EMG_DIVERGED; st->done = 1; break; }
-      st->prev = res;
-      if (it >= st->max_iter) { st->status = EMG_MAX_ITER_REACHED; st->done = 1; }
-      else st->iter = it + 1;
-      break;
-    }
-    default: break;
-  }
+  il_finish(acc, 0.0, partial, st, step);
 }
 
 // Last node of the loop body: keep looping while not done and below the
@@ -357,9 +519,9 @@ __global__ void k_il_host_control(IlState* st) {
   st->loops = st->loops + 1;
 }
 
-__global__ void k_il_start(int64_t n, const double* __restrict__ b, double* __restrict__ x, double* __restrict__ r,
+__global__ void __launch_bounds__(kIlThreads) k_il_start(int64_t n, const double* __restrict__ b, double* __restrict__ x, double* __restrict__ r,
                            double* __restrict__ rh, double* __restrict__ p, double* __restrict__ v, double* partial,
-                           int bicg) {
+                           IlState* st, int bicg) {
   double acc = 0.0;
   for (int64_t i = gtid(); i < n; i += gsize()) {
     const double bi = b[i];
@@ -368,7 +530,7 @@ __global__ void k_il_start(int64_t n, const double* __restrict__ b, double* __re
     if (bicg) { rh[i] = bi; p[i] = bi; v[i] = 0.0; }
     acc += bi * bi;
   }
-  write_partials(acc, 0.0, partial);
+  il_finish(acc, 0.0, partial, st, kInitB);
 }
 
 __global__ void k_il_copy(int64_t n, const double* __restrict__ a, double* __restrict__ b) {
@@ -391,6 +553,8 @@ struct IluState {
   std::vector<int32_t> lptr, uptr;  // level offsets into lrows / urows
   double *x = nullptr, *r = nullptr, *z = nullptr, *p = nullptr, *q = nullptr, *y = nullptr;
   double *rh = nullptr, *v = nullptr, *s = nullptr, *t = nullptr, *part = nullptr;
+  IlSweep lsw, usw;                  // level-order copies for the one-block solves (nchunk 0: not used)
+  double *ypos = nullptr, *zpos = nullptr;
   IlState* st = nullptr;
   cudaStream_t cap = nullptr;
   cudaGraphExec_t loop[2] = {nullptr, nullptr};  // CG, BiCGSTAB
@@ -416,6 +580,87 @@ int ilu_alloc(IluState& s, T** p, int64_t count) {
   EMG_CK(cudaMalloc(&m, sizeof(T) * static_cast<size_t>(std::max<int64_t>(count, 1))));
   s.mem.push_back(m);
   *p = static_cast<T*>(m);
+  return EMG_SUCCESS;
+}
+
+template <class T>
+int ilu_upload(IluState& s, T** dst, const std::vector<T>& v, cudaStream_t st) {
+  int rc = ilu_alloc(s, dst, static_cast<int64_t>(v.size()));
+  if (rc) return rc;
+  if (!v.empty()) EMG_CK(cudaMemcpyAsync(*dst, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice, st));
+  EMG_CK(cudaStreamSynchronize(st));
+  return EMG_SUCCESS;
+}
+
+// The level-order copies of the two triangles for k_ilu_sweeps.
+int ilu_sweeps(IluState& s, const std::vector<int32_t>& rp, const std::vector<int32_t>& col,
+               const std::vector<int32_t>& diag, std::vector<int32_t>& lrows, std::vector<int32_t>& urows,
+               cudaStream_t st) {
+  const int64_t n = s.n;
+  if (n > kIlMaxRows * static_cast<int64_t>(s.lptr.size() - 1) ||
+      std::max(s.lptr.size(), s.uptr.size()) > static_cast<size_t>(kIlMaxLevels))
+    return EMG_SUCCESS;
+  std::vector<int32_t> lpos(n);
+  int rc = EMG_SUCCESS;
+  for (int up = 0; up < 2; ++up) {
+    const std::vector<int32_t>& ptr = up ? s.uptr : s.lptr;
+    std::vector<int32_t>& rows = up ? urows : lrows;
+    IlSweep& S = up ? s.usw : s.lsw;
+    std::vector<int32_t> at(n), lev(1, 0), off(1, 0), in, row, pos, src;
+    S.nlev = static_cast<int32_t>(ptr.size()) - 1;
+    auto count = [&](int32_t i) { return up ? rp[i + 1] - diag[i] - 1 : diag[i] - rp[i]; };
+    for (int32_t l = 0; l < S.nlev; ++l) {  // a level's longest rows first: chunks of even rows
+      std::stable_sort(rows.begin() + ptr[l], rows.begin() + ptr[l + 1],
+                       [&](int32_t a, int32_t b) { return count(a) > count(b); });
+      for (int32_t k = ptr[l]; k < ptr[l + 1]; ++k) {
+        if ((k - ptr[l]) % 32 == 0) row.resize((row.size() + 31) / 32 * 32, -1);
+        at[rows[k]] = static_cast<int32_t>(row.size());
+        row.push_back(rows[k]);
+      }
+      row.resize((row.size() + 31) / 32 * 32, -1);
+      lev.push_back(static_cast<int32_t>(row.size() / 32));
+    }
+    S.nchunk = static_cast<int32_t>(row.size() / 32);
+    in.assign(row.size(), -1);
+    std::vector<int32_t> level_end(S.nchunk);  // first chunk past the chunk's level
+    for (int32_t l = 0; l < S.nlev; ++l)
+      for (int32_t c = lev[l]; c < lev[l + 1]; ++c) level_end[c] = lev[l + 1];
+    for (int32_t c = 0; c < S.nchunk; ++c) {
+      int32_t len = 0;
+      for (int q = 0; q < 32; ++q) {
+        const int32_t i = row[32 * c + q];
+        if (i < 0) continue;
+        len = std::max(len, count(i));
+        in[32 * c + q] = up ? lpos[i] : i;
+      }
+      len = (len + 3) / 4;
+      const size_t base = pos.size();  // [group][lane][4]
+      pos.resize(base + 128 * static_cast<size_t>(len));
+      src.resize(pos.size(), -1);
+      for (int q = 0; q < 32; ++q) {
+        const int32_t i = row[32 * c + q];
+        const int32_t b = i < 0 ? 0 : up ? diag[i] + 1 : rp[i], e = i < 0 ? 0 : up ? rp[i + 1] : diag[i];
+        for (int32_t j = 0; j < 4 * len; ++j) {
+          const size_t k = base + 128 * static_cast<size_t>(j / 4) + 4 * q + j % 4;
+          const int32_t p = b + j < e ? at[col[b + j]] : 32 * c + q;
+          pos[k] = p >= 32 * level_end[c] - kIlRing ? p % kIlRing : ~p;
+          src[k] = b + j < e ? b + j : -1;
+        }
+      }
+      off.push_back(static_cast<int32_t>(pos.size() / 128));
+    }
+    if (!up) lpos = at;
+    if ((rc = ilu_upload(s, &S.lev, lev, st)) || (rc = ilu_upload(s, &S.off, off, st)) ||
+        (rc = ilu_upload(s, &S.in, in, st)) || (rc = ilu_upload(s, &S.row, row, st)) ||
+        (rc = ilu_upload(s, reinterpret_cast<int32_t**>(&S.pos), pos, st)) || (rc = ilu_upload(s, &S.src, src, st)) ||
+        (rc = ilu_alloc(s, &S.val, static_cast<int64_t>(pos.size()) / 2)) ||
+        (rc = ilu_alloc(s, up ? &s.zpos : &s.ypos, 32 * static_cast<int64_t>(S.nchunk))))
+      return rc;
+    if (up && (rc = ilu_alloc(s, &S.dinv, 32 * static_cast<int64_t>(S.nchunk)))) return rc;
+    S.groups = static_cast<int64_t>(pos.size()) / 128;
+  }
+  EMG_CK(cudaFuncSetAttribute(k_ilu_sweeps, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              static_cast<int>(ilu_sweep_smem(kIlMaxLevels, kIlMaxLevels))));
   return EMG_SUCCESS;
 }
 
@@ -467,7 +712,7 @@ int ilu_symbolic(DevCsr& A, IluState& s, cudaStream_t st) {
   EMG_CK(cudaMemcpyAsync(s.lrows, lrows.data(), sizeof(int32_t) * n, cudaMemcpyHostToDevice, st));
   EMG_CK(cudaMemcpyAsync(s.urows, urows.data(), sizeof(int32_t) * n, cudaMemcpyHostToDevice, st));
   EMG_CK(cudaStreamSynchronize(st));
-  return EMG_SUCCESS;
+  return ilu_sweeps(s, rp, col, diag, lrows, urows, st);
 }
 
 int ilu_numeric(DevCsr& A, IluState& s, cudaStream_t st) {
@@ -483,11 +728,21 @@ int ilu_numeric(DevCsr& A, IluState& s, cudaStream_t st) {
   EMG_CK(cudaMemcpyAsync(&f, s.flag, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
   EMG_CK(cudaStreamSynchronize(st));
   s.failed = f != 0;
+  if (!s.failed && s.lsw.nchunk > 0) {
+    k_ilu_pack<<<kIlGrid, kIlThreads, 0, st>>>(s.lsw, s.lu, s.diag);
+    k_ilu_pack<<<kIlGrid, kIlThreads, 0, st>>>(s.usw, s.lu, s.diag);
+    EMG_CK(cudaGetLastError());
+  }
   return EMG_SUCCESS;
 }
 
 // out = U^-1 L^-1 in (out and s.y are work vectors; in is left unchanged)
 void ilu_apply(DevCsr& A, IluState& s, const double* in, double* out, cudaStream_t st) {
+  if (s.lsw.nchunk > 0) {
+    k_ilu_sweeps<<<1, 32 * kIlWarps, ilu_sweep_smem(s.lsw.nlev, s.usw.nlev), st>>>(s.lsw, s.usw, in, s.ypos, s.zpos,
+                                                                                   out, s.st);
+    return;
+  }
   for (size_t k = 0; k + 1 < s.lptr.size(); ++k) {
     const int32_t cnt = s.lptr[k + 1] - s.lptr[k];
     k_ilu_lower<<<level_grid(cnt, kIlLanes), kIlThreads, 0, st>>>(s.lrows + s.lptr[k], cnt, A.row_ptr, A.col, s.diag,
@@ -504,28 +759,22 @@ void ilu_apply(DevCsr& A, IluState& s, const double* in, double* out, cudaStream
 void ilu_body(DevCsr& A, IluState& s, bool bicg, cudaStream_t st) {
   const int64_t n = A.n;
   if (!bicg) {
-    k_il_spmv<<<kIlGrid, kIlThreads, 0, st>>>(n, A.row_ptr, A.col, A.val, s.p, s.q, s.p, nullptr, s.part, s.st);
-    k_il_step<<<1, kIlThreads, 0, st>>>(s.part, kIlGrid, s.st, kCgPq);
-    k_il_cg_xr<<<kIlGrid, kIlThreads, 0, st>>>(n, s.x, s.r, s.p, s.q, s.part, s.st);
-    k_il_step<<<1, kIlThreads, 0, st>>>(s.part, kIlGrid, s.st, kCgRr);
+    k_il_spmv<<<kIlGrid, kIlThreads, 0, st>>>(n, A.row_ptr, A.col, A.val, s.p, s.q, s.p, nullptr, s.part, s.st, kCgPq);
+    k_il_cg_xr<<<kIlGrid, kIlThreads, 0, st>>>(n, s.x, s.r, s.p, s.q, s.part, s.st, kCgRr);
     ilu_apply(A, s, s.r, s.z, st);
-    k_il_dot<<<kIlGrid, kIlThreads, 0, st>>>(n, s.r, s.z, s.part, s.st);
-    k_il_step<<<1, kIlThreads, 0, st>>>(s.part, kIlGrid, s.st, kCgRz);
+    k_il_dot<<<kIlGrid, kIlThreads, 0, st>>>(n, s.r, s.z, s.part, s.st, kCgRz);
     k_il_cg_dir<<<kIlGrid, kIlThreads, 0, st>>>(n, s.p, s.z, s.st);
   } else {
-    k_il_dot<<<kIlGrid, kIlThreads, 0, st>>>(n, s.r, s.rh, s.part, s.st);
-    k_il_step<<<1, kIlThreads, 0, st>>>(s.part, kIlGrid, s.st, kBiRho);
+    k_il_dot<<<kIlGrid, kIlThreads, 0, st>>>(n, s.r, s.rh, s.part, s.st, kBiRho);
     k_il_bi_p<<<kIlGrid, kIlThreads, 0, st>>>(n, s.p, s.r, s.v, s.st);
-    k_il_spmv<<<kIlGrid, kIlThreads, 0, st>>>(n, A.row_ptr, A.col, A.val, s.p, s.v, s.rh, nullptr, s.part, s.st);
-    k_il_step<<<1, kIlThreads, 0, st>>>(s.part, kIlGrid, s.st, kBiRv);
-    k_il_bi_s<<<kIlGrid, kIlThreads, 0, st>>>(n, s.s, s.r, s.v, s.part, s.st);
-    k_il_step<<<1, kIlThreads, 0, st>>>(s.part, kIlGrid, s.st, kBiSs);
+    k_il_spmv<<<kIlGrid, kIlThreads, 0, st>>>(n, A.row_ptr, A.col, A.val, s.p, s.v, s.rh, nullptr, s.part, s.st,
+                                              kBiRv);
+    k_il_bi_s<<<kIlGrid, kIlThreads, 0, st>>>(n, s.s, s.r, s.v, s.part, s.st, kBiSs);
     k_il_bi_early<<<kIlGrid, kIlThreads, 0, st>>>(n, s.x, s.p, s.st);
     ilu_apply(A, s, s.s, s.z, st);
-    k_il_spmv<<<kIlGrid, kIlThreads, 0, st>>>(n, A.row_ptr, A.col, A.val, s.z, s.t, nullptr, s.z, s.part, s.st);
-    k_il_step<<<1, kIlThreads, 0, st>>>(s.part, kIlGrid, s.st, kBiTt);
-    k_il_bi_xr<<<kIlGrid, kIlThreads, 0, st>>>(n, s.x, s.r, s.p, s.z, s.s, s.t, s.part, s.st);
-    k_il_step<<<1, kIlThreads, 0, st>>>(s.part, kIlGrid, s.st, kBiRr);
+    k_il_spmv<<<kIlGrid, kIlThreads, 0, st>>>(n, A.row_ptr, A.col, A.val, s.z, s.t, nullptr, s.z, s.part, s.st,
+                                              kBiTt);
+    k_il_bi_xr<<<kIlGrid, kIlThreads, 0, st>>>(n, s.x, s.r, s.p, s.z, s.s, s.t, s.part, s.st, kBiRr);
   }
 }
 
@@ -625,16 +874,13 @@ int ilu_solve(DevCsr& A, const double* b, double* x, const emg_krylov_config& cf
   init.prev = 1.0;
   init.loop_limit = std::max(cfg.max_iterations, 0) + 2;
   EMG_CK(cudaMemcpyAsync(s.st, &init, sizeof(IlState), cudaMemcpyHostToDevice, st));
-  k_il_start<<<kIlGrid, kIlThreads, 0, st>>>(n, b, s.x, s.r, s.rh, s.p, s.v, s.part, bicg ? 1 : 0);
-  k_il_step<<<1, kIlThreads, 0, st>>>(s.part, kIlGrid, s.st, kInitB);
+  k_il_start<<<kIlGrid, kIlThreads, 0, st>>>(n, b, s.x, s.r, s.rh, s.p, s.v, s.part, s.st, bicg ? 1 : 0);
   if (!bicg) {  // z = M^-1 r, p = z, rz = r.z
     ilu_apply(A, s, s.r, s.z, st);
     k_il_copy<<<kIlGrid, kIlThreads, 0, st>>>(n, s.z, s.p);
-    k_il_dot<<<kIlGrid, kIlThreads, 0, st>>>(n, s.r, s.z, s.part, s.st);
-    k_il_step<<<1, kIlThreads, 0, st>>>(s.part, kIlGrid, s.st, kInitCg);
+    k_il_dot<<<kIlGrid, kIlThreads, 0, st>>>(n, s.r, s.z, s.part, s.st, kInitCg);
   } else {
-    k_il_dot<<<kIlGrid, kIlThreads, 0, st>>>(n, s.r, s.rh, s.part, s.st);
-    k_il_step<<<1, kIlThreads, 0, st>>>(s.part, kIlGrid, s.st, kInitBi);
+    k_il_dot<<<kIlGrid, kIlThreads, 0, st>>>(n, s.r, s.rh, s.part, s.st, kInitBi);
   }
   EMG_CK(cudaGetLastError());
   IlState h;
