@@ -76,6 +76,7 @@ struct Sell {
   bool narrow = false;           // dcol in use (col freed): 10 bytes per slot instead of 12
   int32_t* col = nullptr;        // permuted column of every slot
   int32_t* src = nullptr;        // CSR index of every slot, -1 = padding
+  int32_t* ocol = nullptr;       // column of every slot in the matrix's own numbering (products, csr_spmv)
   double* val = nullptr;
   uint64_t version = ~uint64_t(0);
   int grid = 0;                  // autotuned grid of the register-pipeline SpMV kernels (0: one resident wave)
@@ -630,12 +631,13 @@ __device__ __forceinline__ bool reduce_partials(const double (&vals)[kVals], dou
 }
 
 // ------------------------------------------------------------ SELL build ----
-// Warp per slice: column index (permuted) and CSR source of every slot; rows
-// at or past n are all padding.
+// Warp per slice: column index (permuted), CSR source and, for products in the
+// matrix's own numbering (ocol not null), own column of every slot; rows at or
+// past n are all padding.
 __global__ void k_sell_fill(int64_t n, int64_t nslices, const int64_t* __restrict__ sp,
                             const int32_t* __restrict__ perm, const int32_t* __restrict__ iperm,
                             const int32_t* __restrict__ rp, const int32_t* __restrict__ ccol,
-                            int32_t* __restrict__ col, int32_t* __restrict__ src) {
+                            int32_t* __restrict__ col, int32_t* __restrict__ src, int32_t* __restrict__ ocol) {
   const int lane = threadIdx.x & 31;
   const int64_t warp = gtid() >> 5, nwarps = gstride() >> 5;
   for (int64_t s = warp; s < nslices; s += nwarps) {
@@ -653,6 +655,7 @@ __global__ void k_sell_fill(int64_t n, int64_t nslices, const int64_t* __restric
     for (int j = 0; j < len; ++j) {
       const int64_t k = b0 + static_cast<int64_t>(kGroupStride) * j + lane;
       const int64_t kc = EMG_SELL_PACKED ? packed_col_index(k) : k;
+      if (ocol) ocol[k] = j < rl ? ccol[a + j] : 0;
       if (j < rl) {
         col[kc] = iperm[ccol[a + j]];
         src[k] = a + j;
@@ -800,6 +803,22 @@ __global__ void k_gather(int64_t n, const int32_t* __restrict__ perm, const doub
 __global__ void k_scatter(int64_t n, const int32_t* __restrict__ perm, const double* __restrict__ in,
                           double* __restrict__ out) {
   for (int64_t i = gtid(); i < n; i += gstride()) out[perm[i]] = in[i];
+}
+
+// y = A x in the matrix's own numbering: the slots' own columns and rows
+// written through the permutation, so a product is one launch.  (Gathering x
+// into the solvers' numbering and scattering y out of it took three launches
+// and a memset: 13.4 us for 990 rows and 65 us for the 64^3 matrix.)
+__global__ void __launch_bounds__(kThreads) k_product(Sell A, const int32_t* __restrict__ perm,
+                                                      const double* __restrict__ x, double* __restrict__ y) {
+  A.col = A.ocol;
+  sell_rows<false>(A, x, [&](int64_t row, double s) { y[perm[row]] = s; });
+}
+
+__global__ void k_sell_own_columns(int64_t slots, const int32_t* __restrict__ src, const int32_t* __restrict__ ccol,
+                                   int32_t* __restrict__ ocol) {
+  // padding multiplies column 0 by 0, as the masked entries past a row's end do
+  for (int64_t i = gtid(); i < slots; i += gstride()) ocol[i] = src[i] >= 0 ? ccol[src[i]] : 0;
 }
 
 template <int kMode>
@@ -1388,7 +1407,7 @@ int grid_size() {
 
 // Host: permutation sorting rows by length inside windows (stable), slice
 // offsets; device: slots.
-int build_sell(DevCsr& A, cudaStream_t st) {
+int build_sell(DevCsr& A, bool own_columns, cudaStream_t st) {
   if (!A.sell) A.sell = new Sell();
   Sell& S = *A.sell;
   const int64_t n = A.n;
@@ -1424,6 +1443,7 @@ int build_sell(DevCsr& A, cudaStream_t st) {
   const size_t ns = static_cast<size_t>(std::max<int64_t>(S.slots, 1));
   EMG_CK(cudaMallocAsync(&iperm, sizeof(int32_t) * n, st));
   EMG_CK(cudaMallocAsync(&S.src, sizeof(int32_t) * ns, st));
+  if (own_columns) EMG_CK(cudaMallocAsync(&S.ocol, sizeof(int32_t) * ns, st));
   if (EMG_SELL_PACKED) {  // one buffer: 32-slot chunks of values then columns
     EMG_CK(cudaMallocAsync(&S.val, (sizeof(double) + sizeof(int32_t)) * ns, st));
     S.col = reinterpret_cast<int32_t*>(S.val);
@@ -1434,7 +1454,7 @@ int build_sell(DevCsr& A, cudaStream_t st) {
   k_invert_perm<<<g, kThreads, 0, st>>>(n, S.perm, iperm);
   // every slot of every group is written: slices past the last row are padding
   k_sell_fill<<<g, kThreads, 0, st>>>(n, S.ngroups * kGroup, S.slice_ptr, S.perm, iperm, A.row_ptr, A.col, S.col,
-                                      S.src);
+                                      S.src, S.ocol);
   EMG_CK(cudaGetLastError());
   EMG_CK(cudaFreeAsync(iperm, st));
   S.version = ~uint64_t(0);
@@ -1524,10 +1544,11 @@ int build_sell(DevCsr& A, cudaStream_t st) {
 
 void tune_sell_grid(DevCsr& A, cudaStream_t st);
 
-int ensure_sell(DevCsr& A, cudaStream_t st) {
+// own_columns: products in the matrix's own numbering (csr_spmv) will be asked for
+int ensure_sell(DevCsr& A, cudaStream_t st, bool own_columns = false) {
   bool fresh = false;
   if (!A.sell) {
-    int rc = build_sell(A, st);
+    int rc = build_sell(A, own_columns, st);
     if (rc) return rc;
     fresh = true;
   }
@@ -1545,7 +1566,7 @@ void free_sell(Sell* s) {
   if (!s) return;
   void* col = static_cast<void*>(s->col) == static_cast<void*>(s->val) ? nullptr : static_cast<void*>(s->col);
   for (void* p : {static_cast<void*>(s->perm), static_cast<void*>(s->slice_ptr), col,
-                  static_cast<void*>(s->dcol), static_cast<void*>(s->src), static_cast<void*>(s->val)})
+                  static_cast<void*>(s->dcol), static_cast<void*>(s->src), static_cast<void*>(s->ocol), static_cast<void*>(s->val)})
     if (p) cudaFreeAsync(p, 0);
   delete s;
 }
@@ -2069,16 +2090,21 @@ int csr_spmv(DevCsr& A, const double* x, double* y, cudaStream_t st) {
   if (!x || !y) { set_error("null vector"); return EMG_INVALID_INPUT; }
   int rc = ensure_ws(A, false, 1, st);
   if (rc) return rc;
-  rc = ensure_sell(A, st);
+  rc = ensure_sell(A, st, true);
   if (rc) return rc;
-  const int g = grid_size();
-  const Sell& S = *A.sell;
-  // the workspace vectors hold the permuted operands
-  k_gather<<<g, kThreads, 0, st>>>(A.n, S.perm, x, A.ws->p);
-  int32_t* err = &A.ws->state->copy_err;
-  EMG_CK(cudaMemsetAsync(err, 0, sizeof(int32_t), st));
-  EMG_LAUNCH_SPMV(k_spmv, S, g, st, S, A.ws->p, A.ws->q, err);
-  k_scatter<<<g, kThreads, 0, st>>>(A.n, S.perm, A.ws->q, y);
+  Sell& S = *A.sell;
+  if (!S.ocol && S.slots > 0) {  // built by a solver
+    EMG_CK(cudaMallocAsync(&S.ocol, sizeof(int32_t) * S.slots, st));
+    k_sell_own_columns<<<grid_size(), kThreads, 0, st>>>(S.slots, S.src, A.col, S.ocol);
+  }
+  const int64_t warps = std::max<int64_t>(S.nslices, 1);
+  const int grid = static_cast<int>(std::min<int64_t>(sell_grid<k_product>(S, grid_size()),
+                                                      (warps + kThreads / 32 - 1) / (kThreads / 32)));
+  if (x < y + A.n && y < x + A.n) {  // the operands overlap: rows are written while others still read x
+    EMG_CK(cudaMemcpyAsync(A.ws->p, x, sizeof(double) * A.n, cudaMemcpyDeviceToDevice, st));
+    x = A.ws->p;
+  }
+  k_product<<<grid, kThreads, 0, st>>>(S, S.perm, x, y);
   EMG_CK(cudaGetLastError());
   return EMG_SUCCESS;
 }
