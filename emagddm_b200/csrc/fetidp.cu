@@ -42,7 +42,6 @@ namespace {
 constexpr int kNB = EMG_FETI_NB;  // panel width of the partial Cholesky
 constexpr int kPivBlock = 4 * kNB;  // block of panels whose trailing columns are updated together
 constexpr int kTile = 64;     // output tile of the rank-k updates
-[[maybe_unused]] constexpr int kKC = 32;  // k-chunk of the FMA (non-tensor-core) rank-k updates
 constexpr double kMinInnerTol = 1e-12;  // floor of a pass's multiplier tolerance
 
 enum : int32_t { kErrPivot = 1, kErrAsm = 2, kErrTc = 4, kErrWait = 8 };
@@ -366,115 +365,92 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 
 constexpr int kGK = 16;  // k-chunk of the tile GEMM
 
-struct TileSmem {
-  double a[2][kGK][kTile];
-  double b[2][kGK][kTile];
-};
-
 // C[0:mr, 0:mc] -= (or, kOverwrite, =) A[0:mr, 0:K] * B[0:mc, 0:K]^T for one
-// 64x64 tile with 64 threads; A, B, C column-major.  Thread (tx, ty) owns rows
-// tx + 8a and columns ty + 8b (8 x 8 registers: 16 shared loads per 64 FMAs,
-// conflict-free); k-chunks of 16 double-buffered with cp.async.
-template <bool kOverwrite = false>
-__device__ __forceinline__ void tile_update(double* __restrict__ C, int64_t ldc, int mr, int mc,
-                                            const double* __restrict__ A, int64_t lda,
-                                            const double* __restrict__ B, int64_t ldb, int K, TileSmem& sm) {
-  const int t = threadIdx.x, tx = t & 7, ty = t >> 3;
-  double acc[8][8];
-#pragma unroll
-  for (int a = 0; a < 8; ++a)
-#pragma unroll
-    for (int b = 0; b < 8; ++b) acc[a][b] = 0.0;
-  const int nk = (K + kGK - 1) / kGK;
-  auto load = [&](int chunk, int buf) {
-    const int k0 = chunk * kGK;
-#pragma unroll
-    for (int c = 0; c < kGK; ++c) {
-      const bool kin = k0 + c < K;
-      const bool va = kin && t < mr, vb = kin && t < mc;
-      cp_async8(&sm.a[buf][c][t], va ? A + t + static_cast<int64_t>(k0 + c) * lda : A, va);
-      cp_async8(&sm.b[buf][c][t], vb ? B + t + static_cast<int64_t>(k0 + c) * ldb : B, vb);
-    }
-    cp_async_commit();
-  };
-  if (nk > 0) load(0, 0);
-  for (int i = 0; i < nk; ++i) {
-    if (i + 1 < nk) {
-      load(i + 1, (i + 1) & 1);
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
-    __syncthreads();
-    const int buf = i & 1;
-#pragma unroll 2
-    for (int c = 0; c < kGK; ++c) {
-      double av[8], bv[8];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) { av[q] = sm.a[buf][c][tx + 8 * q]; bv[q] = sm.b[buf][c][ty + 8 * q]; }
-#pragma unroll
-      for (int x = 0; x < 8; ++x)
-#pragma unroll
-        for (int y = 0; y < 8; ++y) acc[x][y] = fma(av[x], bv[y], acc[x][y]);
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int y = 0; y < 8; ++y) {
-    const int cc = ty + 8 * y;
-    if (cc >= mc) continue;
-#pragma unroll
-    for (int x = 0; x < 8; ++x) {
-      const int rr = tx + 8 * x;
-      if (rr < mr) {
-        if (kOverwrite) C[rr + static_cast<int64_t>(cc) * ldc] = acc[x][y];
-        else C[rr + static_cast<int64_t>(cc) * ldc] -= acc[x][y];
-      }
-    }
-  }
-}
-
-// The same tile product on the FP64 tensor cores: 256 threads, warp w owns
-// rows 8w .. 8w+7 of the tile (eight 8x8 blocks across its 64 columns) and
-// issues mma.sync m8n8k4 FP64 per 4-wide step of k; k-chunks of 16 staged by
-// cp.async, double-buffered, rows padded by 4 doubles so that a fragment
-// load (4 k-rows x 8 rows) hits distinct banks.  16 accumulator doubles a
-// thread instead of 64: four blocks of 256 threads fit an SM.
-#ifndef EMG_FETI_DMMA
-#define EMG_FETI_DMMA 1
-#endif
+// M x 64 tile on the FP64 tensor cores; A, B, C column-major.  256 threads,
+// warps 4 x 2, each (M / 4) x 32 of the tile by mma.sync m16n8k8; k-chunks of
+// 16 staged by cp.async, double-buffered, columns padded by 4 doubles so that
+// a fragment load (4 k-rows x 8 rows) hits distinct banks.  What bounds it is
+// the issue of shared-memory loads beside the tensor work, hence the 16-row
+// fragments (m8n8k4 with a warp on 8 rows x 64 columns took 9 loads for 8
+// products of a quarter the size) and, for larger blocks, M = 128, which also
+// halves the reads of B from L2.  The FP64 pipe is 75 % busy on the largest
+// levels (37 TFLOP/s is its rate; three buffers instead of two changed
+// nothing); the pivot-column updates of the 33^3 direct factor went from 7.6 to
+// 6.9 ms, those of the 64^3 FETI-DP factor from 28.1 to 27.0.
 constexpr int kMmaThreads = 256;
 constexpr int kMmaPad = kTile + 4;
+template <int M>
 struct TileSmemMma {
-  double a[2][kGK][kMmaPad];
+  double a[2][kGK][M + 4];
   double b[2][kGK][kMmaPad];
 };
 
-template <bool kOverwrite = false>
+__device__ __forceinline__ void dmma_16x8x8(double (&d)[4], const double (&a)[4], const double (&b)[2]) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+      "{%0, %1, %2, %3};\n"
+      : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
+      : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
+}
+
+// This warp's part of a product with kK columns of k staged as a[k][row] and
+// b[k][col]: acc[i][j] covers rows r0 + 16 i and columns c0 + 8 j; the lane's
+// entries of it are rows fr, fr + 8 and columns 2 fk, 2 fk + 1.
+template <int MI, int kK, class TA, class TB>
+__device__ __forceinline__ void warp_mma(double (&acc)[MI][4][4], const TA& a, const TB& b, int r0, int c0, int fr,
+                                         int fk) {
+#pragma unroll
+  for (int kk = 0; kk < kK; kk += 8) {
+    double bf[4][2];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      bf[j][0] = b[kk + fk][c0 + 8 * j + fr];
+      bf[j][1] = b[kk + fk + 4][c0 + 8 * j + fr];
+    }
+#pragma unroll
+    for (int i = 0; i < MI; ++i) {
+      const int r = r0 + 16 * i + fr;
+      const double af[4] = {a[kk + fk][r], a[kk + fk][r + 8], a[kk + fk + 4][r], a[kk + fk + 4][r + 8]};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) dmma_16x8x8(acc[i][j], af, bf[j]);
+    }
+  }
+}
+
+template <int M, bool kOverwrite = false>
 __device__ __forceinline__ void tile_update_mma(double* __restrict__ C, int64_t ldc, int mr, int mc,
                                                 const double* __restrict__ A, int64_t lda,
                                                 const double* __restrict__ B, int64_t ldb, int K,
-                                                TileSmemMma& sm) {
+                                                TileSmemMma<M>& sm) {
+  constexpr int MI = M / 64;
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-  double acc[8][2];
+  const int fr = lane >> 2, fk = lane & 3;  // fragment row / k of this lane
+  const int r0 = (M / 4) * (w & 3), c0 = 32 * (w >> 2);
+  double acc[MI][4][4];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) acc[j][0] = acc[j][1] = 0.0;
+  for (int i = 0; i < MI; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) acc[i][j][q] = 0.0;
   const int nk = (K + kGK - 1) / kGK;
   auto load = [&](int chunk, int buf) {
     const int k0 = chunk * kGK;
 #pragma unroll
-    for (int i = 0; i < (kGK * kTile) / kMmaThreads; ++i) {
-      const int e = t + kMmaThreads * i;
-      const int c = e / kTile, r = e - c * kTile;
-      const bool kin = k0 + c < K;
-      const bool va = kin && r < mr, vb = kin && r < mc;
-      cp_async8(&sm.a[buf][c][r], va ? A + r + static_cast<int64_t>(k0 + c) * lda : A, va);
-      cp_async8(&sm.b[buf][c][r], vb ? B + r + static_cast<int64_t>(k0 + c) * ldb : B, vb);
+    for (int i = 0; i < kGK * M / kMmaThreads; ++i) {
+      const int e = t + kMmaThreads * i, c = e / M, r = e % M;
+      const bool v = k0 + c < K && r < mr;
+      cp_async8(&sm.a[buf][c][r], v ? A + r + static_cast<int64_t>(k0 + c) * lda : A, v);
+    }
+#pragma unroll
+    for (int i = 0; i < kGK * kTile / kMmaThreads; ++i) {
+      const int e = t + kMmaThreads * i, c = e / kTile, r = e % kTile;
+      const bool v = k0 + c < K && r < mc;
+      cp_async8(&sm.b[buf][c][r], v ? B + r + static_cast<int64_t>(k0 + c) * ldb : B, v);
     }
     cp_async_commit();
   };
   if (nk > 0) load(0, 0);
-  const int fr = lane >> 2, fk = lane & 3;  // fragment row / k of this lane
   for (int i = 0; i < nk; ++i) {
     if (i + 1 < nk) {
       load(i + 1, (i + 1) & 1);
@@ -483,93 +459,34 @@ __device__ __forceinline__ void tile_update_mma(double* __restrict__ C, int64_t 
       cp_async_wait<0>();
     }
     __syncthreads();
-    const int buf = i & 1;
-#pragma unroll
-    for (int kk = 0; kk < kGK; kk += 4) {
-      const double a = sm.a[buf][kk + fk][8 * w + fr];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) dmma_8x8x4(acc[j], a, sm.b[buf][kk + fk][8 * j + fr]);
-    }
+    warp_mma<MI, kGK>(acc, sm.a[i & 1], sm.b[i & 1], r0, c0, fr, fk);
     __syncthreads();
   }
-  const int rr = 8 * w + fr;
-  if (rr >= mr) return;
 #pragma unroll
-  for (int j = 0; j < 8; ++j)
+  for (int i = 0; i < MI; ++i) {
+    double old[4][4];
 #pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const int cc = 8 * j + 2 * fk + q;
-      if (cc < mc) {
-        if (kOverwrite) C[rr + static_cast<int64_t>(cc) * ldc] = acc[j][q];
-        else C[rr + static_cast<int64_t>(cc) * ldc] -= acc[j][q];
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int r = r0 + 16 * i + fr + 8 * (q >> 1), c = c0 + 8 * j + 2 * fk + (q & 1);
+        old[j][q] = !kOverwrite && r < mr && c < mc ? C[r + static_cast<int64_t>(c) * ldc] : 0.0;
       }
-    }
-}
-#if EMG_FETI_DMMA
-constexpr int kTileThreads = kMmaThreads;
-using TileSmemT = TileSmemMma;
-#define EMG_TILE_UPDATE tile_update_mma
-#else
-constexpr int kTileThreads = 64;
-using TileSmemT = TileSmem;
-#define EMG_TILE_UPDATE tile_update
-#endif
-
-#if !EMG_FETI_DMMA
-// C[0:mr, 0:mc] -= A[0:mr, 0:K] * B[0:mc, 0:K]^T for one 64x64 tile with 256
-// threads (4 x 4 registers each, rows 4*tx.., columns 4*ty..), for small K
-// where the update is bound by the C read-modify-write and wants many
-// threads in flight.
-__device__ __forceinline__ void tile_update_wide(double* __restrict__ C, int64_t ldc, int mr, int mc,
-                                                 const double* __restrict__ A, int64_t lda,
-                                                 const double* __restrict__ B, int64_t ldb, int K,
-                                                 double (*As)[kTile + 1], double (*Bs)[kTile + 1]) {
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  double acc[4][4];
 #pragma unroll
-  for (int a = 0; a < 4; ++a)
+    for (int j = 0; j < 4; ++j)
 #pragma unroll
-    for (int b = 0; b < 4; ++b) acc[a][b] = 0.0;
-  for (int kc = 0; kc < K; kc += kKC) {
-    const int kw = min(kKC, K - kc);
-    __syncthreads();
-    for (int e = threadIdx.x; e < kKC * kTile; e += blockDim.x) {
-      const int c = e / kTile, r = e - c * kTile;
-      const bool ok = c < kw;
-      As[c][r] = (ok && r < mr) ? A[r + static_cast<int64_t>(kc + c) * lda] : 0.0;
-      Bs[c][r] = (ok && r < mc) ? B[r + static_cast<int64_t>(kc + c) * ldb] : 0.0;
-    }
-    __syncthreads();
-#pragma unroll 4
-    for (int c = 0; c < kKC; ++c) {
-      double a[4], b[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) { a[q] = As[c][4 * tx + q]; b[q] = Bs[c][4 * ty + q]; }
-#pragma unroll
-      for (int x = 0; x < 4; ++x)
-#pragma unroll
-        for (int y = 0; y < 4; ++y) acc[x][y] = fma(a[x], b[y], acc[x][y]);
-    }
-  }
-#pragma unroll
-  for (int y = 0; y < 4; ++y) {
-    const int cc = 4 * ty + y;
-    if (cc >= mc) continue;
-#pragma unroll
-    for (int x = 0; x < 4; ++x) {
-      const int rr = 4 * tx + x;
-      if (rr < mr) C[rr + static_cast<int64_t>(cc) * ldc] -= acc[x][y];
-    }
+      for (int q = 0; q < 4; ++q) {
+        const int r = r0 + 16 * i + fr + 8 * (q >> 1), c = c0 + 8 * j + 2 * fk + (q & 1);
+        if (r < mr && c < mc) C[r + static_cast<int64_t>(c) * ldc] = kOverwrite ? acc[i][j][q] : old[j][q] - acc[i][j][q];
+      }
   }
 }
-
-#endif
 
 // Panel rows below the diagonal block: X L_kk^T = F[i, k0:k0+nb], formed as
 // X = F L_kk^-T with the inverse that k_potrf_diag stored above the diagonal:
 // one 64-row tile a CTA, the tile and L_kk^-1 staged in shared memory, the
-// 64 x 64 x 64 product on the FP64 tensor cores (mma m8n8k4, warp w owns
-// rows 8w .. 8w+7), the result written back through shared memory.
+// 64 x 64 x 64 product on the FP64 tensor cores, the result written back
+// through shared memory.
 constexpr size_t kTrsmSmem = sizeof(double) * 2 * kTile * kMmaPad;
 __global__ void __launch_bounds__(kMmaThreads) k_trsm_panel(FrontsDev F, int32_t f0, int32_t k0,
                                                             double* __restrict__ fac) {
@@ -601,20 +518,14 @@ __global__ void __launch_bounds__(kMmaThreads) k_trsm_panel(FrontsDev F, int32_t
   }
   __syncthreads();
   const int lane = t & 31, w = t >> 5, fr = lane >> 2, fk = lane & 3;
-  double acc[8][2];
-#pragma unroll
-  for (int j = 0; j < 8; ++j) acc[j][0] = acc[j][1] = 0.0;
-#pragma unroll 4
-  for (int kk = 0; kk < kTile; kk += 4) {
-    const double a = As[kk + fk][8 * w + fr];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) dmma_8x8x4(acc[j], a, Bs[kk + fk][8 * j + fr]);
-  }
+  const int w0 = 16 * (w & 3), wc = 32 * (w >> 2);
+  double acc[1][4][4] = {};
+  warp_mma<1, kTile>(acc, As, Bs, w0, wc, fr, fk);
   __syncthreads();
 #pragma unroll
-  for (int j = 0; j < 8; ++j)
+  for (int j = 0; j < 4; ++j)
 #pragma unroll
-    for (int q = 0; q < 2; ++q) As[8 * j + 2 * fk + q][8 * w + fr] = acc[j][q];
+    for (int q = 0; q < 4; ++q) As[wc + 8 * j + 2 * fk + (q & 1)][w0 + fr + 8 * (q >> 1)] = acc[0][j][q];
   __syncthreads();
   for (int e = t; e < kTile * nb; e += kMmaThreads) {
     const int c = e / kTile, r = e - c * kTile;
@@ -627,59 +538,53 @@ __global__ void __launch_bounds__(kMmaThreads) k_trsm_panel(FrontsDev F, int32_t
 // 64-column panel the rest of its 256-column block, after each block the
 // columns beyond it with K = 256 -- so the trailing columns are read and
 // written once per block instead of once per panel.
-__global__ void __launch_bounds__(256) k_update_pivcols(FrontsDev F, int32_t f0, int32_t ka, int32_t kw,
-                                                        int32_t clo, int32_t chi, double* __restrict__ fac) {
-#if EMG_FETI_DMMA
-  __shared__ TileSmemMma sm;
-#else
-  __shared__ double As[kKC][kTile + 1];
-  __shared__ double Bs[kKC][kTile + 1];
-#endif
+template <int M>
+__global__ void __launch_bounds__(kMmaThreads) k_update_pivcols(FrontsDev F, int32_t f0, int32_t ka, int32_t kw,
+                                                                int32_t clo, int32_t chi,
+                                                                double* __restrict__ fac) {
+  extern __shared__ double tile_sm[];
+  TileSmemMma<M>& sm = *reinterpret_cast<TileSmemMma<M>*>(tile_sm);
   const int32_t k = f0 + blockIdx.y;
   const int32_t np = F.npiv[k];
   if (ka >= np) return;
   const int32_t nb = min(kw, np - ka), fs = F.f[k];
   const int32_t c0 = clo, c1 = min(chi, np);
   if (c0 >= c1) return;
-  const int32_t nct = (c1 - c0 + kTile - 1) / kTile, nrt = (fs - c0 + kTile - 1) / kTile;
+  const int32_t nct = (c1 - c0 + kTile - 1) / kTile, nrt = (fs - c0 + M - 1) / M;
   const int32_t t = blockIdx.x;
   if (t >= nct * nrt) return;
   const int32_t tc = t % nct, tr = t / nct;
-  const int32_t cs = c0 + tc * kTile, rs = c0 + tr * kTile;
-  if (rs + kTile <= cs) return;  // strictly above the diagonal
-  const int mc = min(kTile, c1 - cs), mr = min(kTile, fs - rs);
+  const int32_t cs = c0 + tc * kTile, rs = c0 + tr * M;
+  if (rs + M <= cs) return;  // strictly above the diagonal
+  const int mc = min(kTile, c1 - cs), mr = min(M, fs - rs);
   double* A = fac + F.fac[k];
-#if EMG_FETI_DMMA
-  static_assert(kMmaThreads == 256, "k_update_pivcols runs 256 threads");
-  tile_update_mma(A + rs + static_cast<int64_t>(cs) * fs, fs, mr, mc, A + rs + static_cast<int64_t>(ka) * fs, fs,
-                  A + cs + static_cast<int64_t>(ka) * fs, fs, nb, sm);
-#else
-  tile_update_wide(A + rs + static_cast<int64_t>(cs) * fs, fs, mr, mc, A + rs + static_cast<int64_t>(ka) * fs, fs,
-                   A + cs + static_cast<int64_t>(ka) * fs, fs, nb, As, Bs);
-#endif
+  tile_update_mma<M>(A + rs + static_cast<int64_t>(cs) * fs, fs, mr, mc, A + rs + static_cast<int64_t>(ka) * fs, fs,
+                     A + cs + static_cast<int64_t>(ka) * fs, fs, nb, sm);
 }
 
-// Update block: U -= L21 L21^T (lower tiles), K = npiv.
-__global__ void __launch_bounds__(kTileThreads) k_syrk_update(FrontsDev F, int32_t f0,
-                                                              const double* __restrict__ fac,
-                                                              double* __restrict__ upd) {
-  __shared__ TileSmemT sm;
+// Update block: U -= L21 L21^T (tiles on and below the diagonal), K = npiv.
+template <int M>
+__global__ void __launch_bounds__(kMmaThreads) k_syrk_update(FrontsDev F, int32_t f0,
+                                                             const double* __restrict__ fac,
+                                                             double* __restrict__ upd) {
+  extern __shared__ double tile_sm[];
+  TileSmemMma<M>& sm = *reinterpret_cast<TileSmemMma<M>*>(tile_sm);
+  constexpr int S = M / kTile;  // column tiles per row tile
   const int32_t k = f0 + blockIdx.y;
   const int32_t np = F.npiv[k], fs = F.f[k], nu = fs - np;
   if (nu <= 0) return;
-  const int32_t nt = (nu + kTile - 1) / kTile;
+  // tile t -> (tr, tc), tc < S (tr + 1): S (tr (tr + 1) / 2) tiles before row tr
   const int32_t t = blockIdx.x;
-  if (t >= nt * (nt + 1) / 2) return;
-  // t -> lower tile (tr >= tc), t = tr (tr + 1) / 2 + tc
-  int32_t tr = static_cast<int32_t>((sqrt(8.0 * t + 1.0) - 1.0) * 0.5);
-  while ((tr + 1) * (tr + 2) / 2 <= t) ++tr;
-  while (tr * (tr + 1) / 2 > t) --tr;
-  const int32_t tc = t - tr * (tr + 1) / 2;
-  const int32_t rs = tr * kTile, cs = tc * kTile;
-  const int mr = min(kTile, nu - rs), mc = min(kTile, nu - cs);
+  int32_t tr = static_cast<int32_t>((sqrt(8.0 * (t / S) + 1.0) - 1.0) * 0.5);
+  while (S * ((tr + 1) * (tr + 2) / 2) <= t) ++tr;
+  while (S * (tr * (tr + 1) / 2) > t) --tr;
+  const int32_t tc = t - S * (tr * (tr + 1) / 2);
+  const int32_t rs = tr * M, cs = tc * kTile;
+  if (rs >= nu || cs >= nu) return;
+  const int mr = min(M, nu - rs), mc = min(kTile, nu - cs);
   const double* L = fac + F.fac[k];
   double* U = upd + F.upd[k];
-  EMG_TILE_UPDATE(U + rs + static_cast<int64_t>(cs) * nu, nu, mr, mc, L + np + rs, fs, L + np + cs, fs, np, sm);
+  tile_update_mma<M>(U + rs + static_cast<int64_t>(cs) * nu, nu, mr, mc, L + np + rs, fs, L + np + cs, fs, np, sm);
 }
 
 // Mixed-precision variants of the two contractions of the factor (the
@@ -755,14 +660,14 @@ __global__ void __launch_bounds__(tc::kThreads) k_tc_tile_test(double* C, int64_
 //   k_trtri_off:   one CTA per column block J (J-major order, so the longest
 //                  chains start first), row blocks I = J+1, J+2, ... in order:
 //                  X_IJ = -X_II (sum_{J<=K<I} L_IK X_KJ), the sum a 64-wide
-//                  tile product on the FP64 tensor cores (mma m8n8k4, k-chunks
+//                  tile product on the FP64 tensor cores (k-chunks
 //                  double-buffered by cp.async, X_KJ read from the transposes
 //                  this CTA stored in the upper blocks), the product with
 //                  X_II a second tile product from shared memory; X_IJ and
 //                  its transpose are stored through shared memory, coalesced.
 constexpr int kTB = 64;
 constexpr size_t kTrtriOffSmem = sizeof(double) * 2 * kTB * kMmaPad;
-static_assert(kTB == kTile && sizeof(TileSmemMma) <= kTrtriOffSmem && (kGK * kTB) % kMmaThreads == 0,
+static_assert(kTB == kTile && sizeof(TileSmemMma<kTB>) <= kTrtriOffSmem && (kGK * kTB) % kMmaThreads == 0,
               "staging of the triangular inverse");
 
 __global__ void __launch_bounds__(256) k_trtri_diag(int32_t n_mat, const int32_t* __restrict__ dim,
@@ -797,7 +702,7 @@ __global__ void __launch_bounds__(kMmaThreads) k_trtri_off(int32_t n_mat, const 
                                                            const double* __restrict__ Lbase,
                                                            double* __restrict__ Xbase) {
   extern __shared__ double smd[];
-  TileSmemMma& sm = *reinterpret_cast<TileSmemMma*>(smd);
+  TileSmemMma<kTB>& sm = *reinterpret_cast<TileSmemMma<kTB>*>(smd);
   double (*Ts)[kMmaPad] = reinterpret_cast<double (*)[kMmaPad]>(smd);             // after the sum: T, then X_IJ
   double (*Ds)[kMmaPad] = reinterpret_cast<double (*)[kMmaPad]>(smd + kTB * kMmaPad);  // X_II, k-major
   const int32_t m = blockIdx.x;
@@ -809,6 +714,7 @@ __global__ void __launch_bounds__(kMmaThreads) k_trtri_off(int32_t n_mat, const 
   const double* L = Lbase + l_off[m];
   double* X = Xbase + x_off[m];
   const int t = threadIdx.x, lane = t & 31, w = t >> 5, fr = lane >> 2, fk = lane & 3;
+  const int w0 = 16 * (w & 3), wc = 32 * (w >> 2);
   // right operand B(c, k) = X[c0 + k, c0 + c]: the stored transpose X[c0 + c, c0 + k]
   const double* B = X + c0 + static_cast<int64_t>(c0) * n;
   for (int32_t I = J + 1; I < nb; ++I) {
@@ -829,9 +735,7 @@ __global__ void __launch_bounds__(kMmaThreads) k_trtri_off(int32_t n_mat, const 
       }
       cp_async_commit();
     };
-    double acc[8][2];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) acc[j][0] = acc[j][1] = 0.0;
+    double acc[1][4][4] = {};
     load(0, 0);
     for (int i = 0; i < nk; ++i) {
       if (i + 1 < nk) {
@@ -841,38 +745,28 @@ __global__ void __launch_bounds__(kMmaThreads) k_trtri_off(int32_t n_mat, const 
         cp_async_wait<0>();
       }
       __syncthreads();
-      const int buf = i & 1;
-#pragma unroll
-      for (int kk = 0; kk < kGK; kk += 4) {
-        const double a = sm.a[buf][kk + fk][8 * w + fr];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) dmma_8x8x4(acc[j], a, sm.b[buf][kk + fk][8 * j + fr]);
-      }
+      warp_mma<1, kGK>(acc, sm.a[i & 1], sm.b[i & 1], w0, wc, fr, fk);
       __syncthreads();
     }
     // T = -sum (rows of T are the k of the product with X_II); X_II lower, k-major
 #pragma unroll
-    for (int j = 0; j < 8; ++j)
+    for (int j = 0; j < 4; ++j)
 #pragma unroll
-      for (int q = 0; q < 2; ++q) Ts[8 * w + fr][8 * j + 2 * fk + q] = -acc[j][q];
+      for (int q = 0; q < 4; ++q) {
+        Ts[w0 + fr + 8 * (q >> 1)][wc + 8 * j + 2 * fk + (q & 1)] = -acc[0][j][q];
+        acc[0][j][q] = 0.0;
+      }
     for (int e = t; e < kTB * kTB; e += kMmaThreads) {
       const int k = e / kTB, r = e - k * kTB;
       Ds[k][r] = (r < h && k <= r) ? X[(r0 + r) + static_cast<int64_t>(r0 + k) * n] : 0.0;
     }
     __syncthreads();
-#pragma unroll
-    for (int j = 0; j < 8; ++j) acc[j][0] = acc[j][1] = 0.0;
-#pragma unroll 4
-    for (int kk = 0; kk < kTB; kk += 4) {
-      const double a = Ds[kk + fk][8 * w + fr];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) dmma_8x8x4(acc[j], a, Ts[kk + fk][8 * j + fr]);
-    }
+    warp_mma<1, kTB>(acc, Ds, Ts, w0, wc, fr, fk);
     __syncthreads();
 #pragma unroll
-    for (int j = 0; j < 8; ++j)
+    for (int j = 0; j < 4; ++j)
 #pragma unroll
-      for (int q = 0; q < 2; ++q) Ts[8 * w + fr][8 * j + 2 * fk + q] = acc[j][q];
+      for (int q = 0; q < 4; ++q) Ts[w0 + fr + 8 * (q >> 1)][wc + 8 * j + 2 * fk + (q & 1)] = acc[0][j][q];
     __syncthreads();
     for (int e = t; e < kTB * kTB; e += kMmaThreads) {  // X_IJ, coalesced along its rows
       const int c = e / kTB, r = e - c * kTB;
@@ -1932,10 +1826,11 @@ __global__ void k_face_transpose(FacesDev Fc, const double* __restrict__ X, doub
 }
 
 // C_f = A_f B_f^T for every face (n x n, column-major, same offsets).
-__global__ void __launch_bounds__(kTileThreads) k_face_gemm_nt(FacesDev Fc, const double* __restrict__ A,
+__global__ void __launch_bounds__(kMmaThreads) k_face_gemm_nt(FacesDev Fc, const double* __restrict__ A,
                                                                const double* __restrict__ B,
                                                                double* __restrict__ C) {
-  __shared__ TileSmemT sm;
+  extern __shared__ double tile_sm[];
+  TileSmemMma<kTile>& sm = *reinterpret_cast<TileSmemMma<kTile>*>(tile_sm);
   const int32_t f = blockIdx.y;
   const int32_t n = Fc.dim[f];
   const int32_t nt = (n + kTile - 1) / kTile;
@@ -1945,7 +1840,8 @@ __global__ void __launch_bounds__(kTileThreads) k_face_gemm_nt(FacesDev Fc, cons
   const int32_t rs = tr * kTile, cs = tc * kTile;
   const int mr = min(kTile, n - rs), mc = min(kTile, n - cs);
   const int64_t o = Fc.off[f];
-  EMG_TILE_UPDATE<true>(C + o + rs + static_cast<int64_t>(cs) * n, n, mr, mc, A + o + rs, n, B + o + cs, n, n, sm);
+  tile_update_mma<kTile, true>(C + o + rs + static_cast<int64_t>(cs) * n, n, mr, mc, A + o + rs, n, B + o + cs, n, n,
+                               sm);
 }
 
 // w[e_i] = sum_j D[i, j] sign r[lam_j] for every face side (side = blockIdx.y & 1),
@@ -2570,6 +2466,19 @@ int FetiDP::factor_range(int32_t f0, int32_t f1) {
   if (kTrsmSmem > 48 * 1024 && !capturing)  // (set by the eager factorization before any capture)
     EMG_CK(cudaFuncSetAttribute(k_trsm_panel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 static_cast<int>(kTrsmSmem)));
+  if (!capturing) {
+    EMG_CK(cudaFuncSetAttribute(k_update_pivcols<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                static_cast<int>(sizeof(TileSmemMma<128>))));
+    EMG_CK(cudaFuncSetAttribute(k_syrk_update<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                static_cast<int>(sizeof(TileSmemMma<128>))));
+  }
+  // 128-row tiles where they still fill the GPU (two CTAs an SM): the 64^3
+  // FETI-DP step takes 224.5 ms with the line anywhere from 0 to 1,200 tiles and
+  // 226.8 with 64-row tiles alone, the 33^3 direct step 33.3 and 33.7 (33.6
+  // with 128-row tiles alone)
+  auto tall = [](int32_t rows, int32_t col_tiles, unsigned fronts) {
+    return rows >= 256 && static_cast<int64_t>((rows + 127) / 128) * col_tiles * fronts >= 2 * 148;
+  };
   // mixed precision: the subdomain fronts' contractions on the TF32 tensor cores
   const bool tc_here = tc_factor && f1 <= F;
   if (tc_here && !capturing) {
@@ -2602,16 +2511,18 @@ int FetiDP::factor_range(int32_t f0, int32_t f1) {
       // the rest of this panel's block, then (after its last panel) the columns beyond the block
       const int32_t b0 = (k0 / kPivBlock) * kPivBlock, b1 = b0 + kPivBlock;
       const int32_t c1 = std::min(b1, mnp);
-      if (c0 < c1) {
-        const int32_t nct = (c1 - c0 + kTile - 1) / kTile, nrt = (mf - c0 + kTile - 1) / kTile;
-        k_update_pivcols<<<dim3(static_cast<unsigned>(nct * nrt), active), 256, 0, st>>>(fd, f0, k0, kNB, c0, b1,
-                                                                                          fac_d);
-      }
-      if (c0 == b1 && b1 < mnp) {
-        const int32_t nct = (mnp - b1 + kTile - 1) / kTile, nrt = (mf - b1 + kTile - 1) / kTile;
-        k_update_pivcols<<<dim3(static_cast<unsigned>(nct * nrt), active), 256, 0, st>>>(fd, f0, b0, kPivBlock, b1,
-                                                                                          INT32_MAX, fac_d);
-      }
+      auto update = [&](int32_t ka, int32_t kw, int32_t clo, int32_t cend, int32_t chi) {
+        const int32_t nct = (cend - clo + kTile - 1) / kTile;
+        auto run = [&](auto kernel, int M, size_t smem) {
+          const int32_t nrt = (mf - clo + M - 1) / M;
+          kernel<<<dim3(static_cast<unsigned>(nct * nrt), active), kMmaThreads, smem, st>>>(fd, f0, ka, kw, clo, chi,
+                                                                                            fac_d);
+        };
+        if (tall(mf - clo, nct, active)) run(k_update_pivcols<128>, 128, sizeof(TileSmemMma<128>));
+        else run(k_update_pivcols<64>, 64, sizeof(TileSmemMma<64>));
+      };
+      if (c0 < c1) update(k0, kNB, c0, c1, b1);
+      if (c0 == b1 && b1 < mnp) update(b0, kPivBlock, b1, mnp, INT32_MAX);
     }
   }
   if (max_nu > 0 && tc_here) {
@@ -2619,8 +2530,13 @@ int FetiDP::factor_range(int32_t f0, int32_t f1) {
     k_syrk_update_tc<<<dim3(static_cast<unsigned>(nt * (nt + 1) / 2), nf), tc::kThreads, tc::kSmemBytes, st>>>(
         fd, f0, fac_d, upd_d, err_d);
   } else if (max_nu > 0) {
-    const int32_t nt = (max_nu + kTile - 1) / kTile;
-    k_syrk_update<<<dim3(static_cast<unsigned>(nt * (nt + 1) / 2), nf), kTileThreads, 0, st>>>(fd, f0, fac_d, upd_d);
+    const int32_t n1 = (max_nu + 63) / 64, n2 = (max_nu + 127) / 128;
+    if (tall(max_nu, n1 / 2, nf))
+      k_syrk_update<128><<<dim3(static_cast<unsigned>(n2 * (n2 + 1)), nf), kMmaThreads, sizeof(TileSmemMma<128>), st>>>(
+          fd, f0, fac_d, upd_d);
+    else
+      k_syrk_update<64><<<dim3(static_cast<unsigned>(n1 * (n1 + 1) / 2), nf), kMmaThreads, sizeof(TileSmemMma<64>),
+                          st>>>(fd, f0, fac_d, upd_d);
   }
   EMG_CK(cudaGetLastError());
   return EMG_SUCCESS;
@@ -2849,9 +2765,9 @@ int FetiDP::setup_deluxe() {
   k_face_transpose<true><<<dim3(blocks_for(f2, 256, 256), nf), 256, 0, st>>>(fc, fX_d, fXt_d);  // (L^-1)^T
   const int32_t nt = (max_fdim + kTile - 1) / kTile;
   const dim3 g(static_cast<unsigned>(nt * nt), nf);
-  k_face_gemm_nt<<<g, kTileThreads, 0, st>>>(fc, fXt_d, fXt_d, fZ_d);   // (S_a + S_b)^-1 = X^T X
-  k_face_gemm_nt<<<g, kTileThreads, 0, st>>>(fc, fZ_d, fSb_d, fDa_d);   // D_a = (S_a + S_b)^-1 S_b
-  k_face_gemm_nt<<<g, kTileThreads, 0, st>>>(fc, fZ_d, fSa_d, fDb_d);   // D_b = (S_a + S_b)^-1 S_a
+  k_face_gemm_nt<<<g, kMmaThreads, sizeof(TileSmemMma<kTile>), st>>>(fc, fXt_d, fXt_d, fZ_d);   // (S_a + S_b)^-1 = X^T X
+  k_face_gemm_nt<<<g, kMmaThreads, sizeof(TileSmemMma<kTile>), st>>>(fc, fZ_d, fSb_d, fDa_d);   // D_a = (S_a + S_b)^-1 S_b
+  k_face_gemm_nt<<<g, kMmaThreads, sizeof(TileSmemMma<kTile>), st>>>(fc, fZ_d, fSa_d, fDb_d);   // D_b = (S_a + S_b)^-1 S_a
   // transposes for the row pass, in the buffers of X and X^T (no longer needed)
   k_face_transpose<false><<<dim3(blocks_for(f2, 256, 256), nf), 256, 0, st>>>(fc, fDa_d, fX_d);
   k_face_transpose<false><<<dim3(blocks_for(f2, 256, 256), nf), 256, 0, st>>>(fc, fDb_d, fXt_d);
