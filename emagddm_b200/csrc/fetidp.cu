@@ -503,18 +503,23 @@ __global__ void __launch_bounds__(kMmaThreads) k_trsm_panel(FrontsDev F, int32_t
   const int32_t h = min(kTile, fs - r0);
   double* A = fac + F.fac[k];
   const int t = threadIdx.x;
-  for (int e = t; e < kTile * kTile; e += kMmaThreads) {
-    const int c = e / kTile, r = e - c * kTile;
-    As[c][r] = (r < h && c < nb) ? A[(r0 + r) + static_cast<int64_t>(k0 + c) * fs] : 0.0;
-  }
-  for (int e = t; e < kTile * kTile; e += kMmaThreads) {
-    const int c = e / kTile, q = e - c * kTile;  // Linv(c, q): stored at row q, column c of the block
-    double v = 0.0;
-    if (c < nb && q < nb) {
-      if (c > q) v = A[(k0 + q) + static_cast<int64_t>(k0 + c) * fs];
-      else if (c == q) v = 1.0 / A[(k0 + c) + static_cast<int64_t>(k0 + c) * fs];
+  {  // both operands' entries all in flight before the first is stored
+    constexpr int N = kTile * kTile / kMmaThreads;
+    const int r = t % kTile, c0 = t / kTile;
+    double va[N], vb[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const int c = c0 + kMmaThreads / kTile * i;
+      va[i] = (r < h && c < nb) ? A[(r0 + r) + static_cast<int64_t>(k0 + c) * fs] : 0.0;
+      // Linv(c, r): stored at row r, column c of the block; 1 / L_cc on its diagonal
+      vb[i] = (c < nb && r <= c) ? A[(k0 + r) + static_cast<int64_t>(k0 + c) * fs] : 0.0;
     }
-    Bs[q][c] = v;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const int c = c0 + kMmaThreads / kTile * i;
+      As[c][r] = va[i];
+      Bs[r][c] = r == c && c < nb ? 1.0 / vb[i] : vb[i];
+    }
   }
   __syncthreads();
   const int lane = t & 31, w = t >> 5, fr = lane >> 2, fk = lane & 3;
