@@ -174,12 +174,14 @@ constexpr double kPivRel = 1e-11;
 
 // The diagonal block (nb <= 64 columns; a narrower last panel is padded with
 // identity rows and columns, which leave the real entries unchanged) in
-// shared memory, 256 threads, as a Cholesky of 16-column sub-panels.  It is a
+// shared memory, 256 threads, as a Cholesky of kPW-column sub-panels.  It is a
 // serial chain, one CTA's latency per panel of every front, so the layout is
-// chosen for the chain: one warp holds the sub-panel's 16 columns in
-// registers (a lane two rows), so a column costs a shuffle of the pivot, one
-// rsqrt and a multiply, with no barrier; all eight warps subtract the
-// rank-16 product from the columns to its right (8 x 8 tiles on the FP64
+// chosen for the chain: one warp holds the sub-panel's columns in
+// registers (a lane two rows), no barrier between columns, and the next
+// pivot a'_cc - a'_c^2 / v is formed from unscaled entries fetched while the
+// root of this one is on its way, so a column costs a reciprocal root and two
+// operations; all eight warps subtract the
+// rank-kPW product from the columns to its right (8 x 8 tiles on the FP64
 // tensor cores), two barriers a sub-panel.  Pivot test against d0, the
 // matrix's own diagonal, when given.  Then X = L^-1: the four 16 x 16
 // diagonal inverses by substitution in registers, a half warp each, and the
@@ -189,7 +191,8 @@ constexpr double kPivRel = 1e-11;
 // one (read by the panel TRSM and the inverse factors), the block is written
 // back in one coalesced pass.  Column-by-column code with three barriers a
 // column took 92 us a launch on the 8 subdomains of the 16^3 mesh and 87 us
-// on the fronts of the 33^3 direct factor; this one 20 and 23 us.
+// on the fronts of the 33^3 direct factor; this one 18 and 21 us.
+constexpr int kPW = 8;  // columns of a sub-panel (16: the unrolled code no longer fits the instruction cache, 21 and 24 us)
 struct PotrfSmem {
   double D[kNB][kNB + 4];    // [column][row]: L at row >= column, X(r, c) at [r][c]
   double T[3][16][20];       // sum_k L_ik X_kj of the blocks of one distance, [blk][k][n]
@@ -201,6 +204,18 @@ __device__ __forceinline__ void dmma_8x8x4(double (&d)[2], double a, double b) {
   asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
                : "+d"(d[0]), "+d"(d[1])
                : "d"(a), "d"(b));
+}
+
+// 1 / sqrt(v) to within an ulp, without the branches of the library's (which
+// keep the columns' chains from overlapping): the hardware's approximation
+// y (22 bits) and one step of third order, y (1 + e / 2 + 3 e^2 / 8) with
+// e = 1 - v y^2.  Denormal pivots take the library's.
+__device__ __forceinline__ double inv_sqrt(double v) {
+  if (__double2hiint(v) < 0x00100000) return rsqrt(v);
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(v));
+  const double e = fma(-(v * y), y, 1.0);
+  return fma(y * e, fma(0.375, e, 0.5), y);
 }
 
 __device__ __forceinline__ void potrf_panel(double* __restrict__ A, int32_t fs, int32_t nb,
@@ -225,53 +240,64 @@ __device__ __forceinline__ void potrf_panel(double* __restrict__ A, int32_t fs, 
     for (int i = 0; i < kNB / 4; ++i) D[(t >> 6) + 4 * i][rr] = v[i];
   }
   __syncthreads();
-  const int np = (nb + 15) / 16;  // sub-panels with real columns; the rest is identity
+  const int np = (nb + 15) / 16;  // 16-column blocks with real columns; the rest is identity
+  const int nw = (nb + kPW - 1) / kPW;
 #pragma unroll 1
-  for (int p = 0; p < np; ++p) {
-    const int c0 = 16 * p, hi = c0 & 32;  // rows hi + lane (and 32 + lane while the pivots are in the first half)
+  for (int p = 0; p < nw; ++p) {
+    const int c0 = kPW * p, hi = c0 & 32;  // rows hi + lane (and 32 + lane while the pivots are in the first half)
     if (w == 0) {
-      double a0[16], a1[16];
+      double a0[kPW], a1[kPW];
 #pragma unroll
-      for (int k = 0; k < 16; ++k) {
+      for (int k = 0; k < kPW; ++k) {
         a0[k] = D[c0 + k][hi + lane];
         a1[k] = hi ? 0.0 : D[c0 + k][32 + lane];
       }
+      double v = __shfl_sync(0xffffffffu, a0[0], c0 & 31);  // the pivot of column c
+      double least[kPW];  // what it has to exceed (identity columns past nb: 0)
 #pragma unroll
-      for (int c = 0; c < 16; ++c) {
-        double v = __shfl_sync(0xffffffffu, a0[c], (c0 + c) & 31);
-        if (c0 + c < nb && (!(v > 0.0) || (d0 && !(v > kPivRel * sm.d0[c0 + c])))) {
-          if (lane == 0) atomicOr(err, kErrPivot);
-          // a unit pivot keeps the rest finite; the factorization is reported as failed
-          if (lane == ((c0 + c) & 31)) a0[c] = 1.0;
-          v = 1.0;
+      for (int c = 0; c < kPW; ++c) least[c] = kPivRel * sm.d0[c0 + c];
+      bool fail = false;
+#pragma unroll
+      for (int c = 0; c < kPW; ++c) {
+        // row c + 1's entries of this column and the next, before the pivot's root is known
+        double p1 = 0.0, pp = 1.0;
+        if (c + 1 < kPW) {
+          p1 = __shfl_sync(0xffffffffu, a0[c], (c0 + c + 1) & 31);
+          pp = __shfl_sync(0xffffffffu, a0[c + 1], (c0 + c + 1) & 31);
         }
-        const double ri = rsqrt(v);
+        const bool bad = !(v > 0.0) || !(v > least[c]);
+        fail |= bad;  // a unit pivot keeps the rest finite; the factorization is reported as failed
+        const double root = inv_sqrt(v), ri = bad ? 1.0 : root;
+        v = bad ? 1.0 : v;
+        if (lane == ((c0 + c) & 31)) a0[c] = v;
         a0[c] *= ri;
         a1[c] *= ri;
         if (lane == 0) sm.rinv[c0 + c] = ri;
+        if (c + 1 < kPW) v = fma(-(p1 * p1), ri * ri, pp);
 #pragma unroll
-        for (int q = c + 1; q < 16; ++q) {
+        for (int q = c + 1; q < kPW; ++q) {
           const double m = __shfl_sync(0xffffffffu, a0[c], (c0 + q) & 31);
           a0[q] -= a0[c] * m;
           a1[q] -= a1[c] * m;
         }
       }
+      if (fail && lane == 0) atomicOr(err, kErrPivot);
 #pragma unroll
-      for (int k = 0; k < 16; ++k) {
+      for (int k = 0; k < kPW; ++k) {
         if (hi + lane >= c0 + k) D[c0 + k][hi + lane] = a0[k];
         if (!hi) D[c0 + k][32 + lane] = a1[k];
       }
     }
     __syncthreads();
     // trailing 8 x 8 tiles (i >= j) of the columns right of the sub-panel
-    const int n8 = 2 * (np - p - 1), b8 = c0 / 8 + 2;
+    const int n8 = kPW / 8 * (nw - p - 1), b8 = (c0 + kPW) / 8;
     for (int e = w; e < n8 * (n8 + 1) / 2; e += 8) {
       int i = 0, base = 0;
       while (base + i + 1 <= e) base += ++i;
       const int r0 = 8 * (b8 + i), q0 = 8 * (b8 + e - base);
       double acc[2] = {0.0, 0.0};
 #pragma unroll
-      for (int kk = 0; kk < 16; kk += 4)
+      for (int kk = 0; kk < kPW; kk += 4)
         dmma_8x8x4(acc, D[c0 + kk + fk][r0 + fr], D[c0 + kk + fk][q0 + fr]);
 #pragma unroll
       for (int q = 0; q < 2; ++q)
