@@ -29,6 +29,7 @@
 #include "device.h"
 #include "fetidp.h"
 #include "fetidp_dev.h"
+#include "sell_tma.cuh"
 #include "tc_tile.cuh"
 #include "trace.h"
 #include "tune.h"
@@ -1557,6 +1558,222 @@ __global__ void __launch_bounds__(512) k_block_colgemv(int32_t n_mat, const int3
   if (lane == 0) y[v_off[m] + c] = acc;
 }
 
+// Products with the roots' triangles in one read of them, row by row (row r:
+// entries 0..r, contiguous as column r of the upper half):
+//   kInverse:  y = L^-T (L^-1 w): z_r = row . w, then y += z_r row while the row
+//              is still at hand, where two column-dot passes read L^-1 twice;
+//   symmetric: y = S w: y_r gets row . w, and y += w_r row left of the diagonal.
+// HBM and the steps' own chain bound both.  Every CTA owns a run of whole rows
+// that may end in one root and start the next; each piece (a TriSeg) keeps its y
+// in registers, kK columns a thread, and writes it to its own slot; k_tri_sum
+// adds a root's slots in order.  kR rows at a time share one block sum (a warp
+// reduce-scatter, then every warp adds the 16 warps' values in the same order:
+// one barrier).  The rows of the next steps are on their way into a ring in
+// shared memory meanwhile, as bulk copies by one thread: 160 to 200 KB in flight
+// an SM without a register or an issue slot of the threads that compute.  A row
+// is copied from the 16-byte boundary at or before its start.  The waits are
+// bounded: one that runs out sets kErrWait, and the product becomes NaN.
+// Split: by entries + kTriRowCost a row.  With the entries alone the CTAs of the
+// short rows take three times as long as the others (64 roots of 1,500 to 3,100
+// unknowns, 1.39 GB: 554 us at 0, 333 at 512, 311 at 1024, 289 at 2048 to 4096).
+// kR: the most rows that the registers hold.
+// Measured against the two column-dot passes / the tile pass (B200):
+//   1.39 GB (64^3 in 64)  L^-T L^-1 w 498 -> 301 us   S w 316 -> 320 us
+//    470 MB (48^3 in 27)              186 -> 126          156 -> 132
+//     75 MB (32^3 in 8)                47 -> 40            76 -> 43
+// 64^3 in 64: multiplier iterations 40.5 -> 33.9 ms, factor and solve 222 -> 212 ms.
+// y's error against 80-bit sums (L^-1 of random matrices with condition 1e3 and
+// 1e4, 900 to 2,500 unknowns): 1.61e-16 to 1.90e-16 of its norm, with the column
+// dots 1.67e-16 to 2.04e-16; without the carried roundings of add_carried it was
+// 1.9e-16 to 3.3e-16.  S w needs none: the tile pass adds a quarter of a row in
+// one chain, here it is 128 sums of kR.
+constexpr int kTriT = 512, kTriMaxK = 8, kTriRing = 24600, kTriStages = 8;
+constexpr int32_t kTriMaxN = kTriT * kTriMaxK;
+constexpr int64_t kTriRowCost = 3072;  // what a row costs beside its entries, in entries
+constexpr int64_t kTriMinRow = 384, kTriMinEntries = 2000000;
+constexpr int kTriRed = 2 * 8 * (kTriT / 32);  // the warps' sums, two buffers
+constexpr size_t kTriSmem = sizeof(double) * (kTriRing + kTriMaxN + kTriRed + kTriStages);
+constexpr int kTriFlush = 16;
+constexpr int kTriPad = 4;  // entries past the last block that a copy rounded up to 16 bytes may read
+
+// (sum, carried roundings) + v: Knuth's exact sum of two numbers.
+__device__ __forceinline__ double2 add_carried(double2 a, double v) {
+  const double s = a.x + v, b = s - a.x;
+  return make_double2(s, a.y + ((a.x - (s - b)) + (v - b)));
+}
+
+struct TriSmem {
+  double *ring, *ws, *red;
+  uint64_t* full;
+};
+
+template <bool kInverse, int kK, int kR, class T>
+__device__ __forceinline__ bool tri_rows(const T* __restrict__ M, int64_t off, int32_t n, int32_t ra, int32_t rb,
+                                         const TriSmem& sm, uint32_t& phase, uint64_t pol,
+                                         double2* __restrict__ out) {
+  static_assert(kR <= 8 && kTriT == 512, "a lane adds kR / 2 of the 16 warps' values");
+  constexpr int V = 16 / sizeof(T);
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  const int cap = (rb + 2 * V - 2) / V * V;  // a row from the boundary before it, whole vectors
+  const int depth = min(kTriStages, static_cast<int>(kTriRing * sizeof(double) / (kR * cap * sizeof(T))));
+  const int steps = (rb - ra + kR - 1) / kR;
+  T* const ring = reinterpret_cast<T*>(sm.ring);
+  auto head = [&](int32_t r) { return static_cast<int>((off + static_cast<int64_t>(r) * n) & (V - 1)); };
+  auto fetch = [&](int i, int stage) {  // one thread: the rows of step i
+    const int32_t r0 = ra + i * kR, r1 = min(r0 + kR, rb);
+    uint32_t bytes = 0;
+    for (int32_t r = r0; r < r1; ++r) bytes += ((r + head(r)) / V + 1) * 16u;
+    tma::mbar_expect_tx(sm.full + stage, bytes);
+    for (int32_t r = r0; r < r1; ++r)
+      tma::bulk_g2s(ring + (stage * kR + (r - r0)) * cap, M + off + static_cast<int64_t>(r) * n - head(r),
+                    ((r + head(r)) / V + 1) * 16u, sm.full + stage, pol);
+  };
+  if (t == 0)
+    for (int i = 0; i < min(depth, steps); ++i) fetch(i, i);
+  double acc[kK] = {};
+  for (int i = 0, stage = 0, buf = 0; i < steps; ++i, buf ^= 1) {
+    const bool ok = tma::mbar_wait(sm.full + stage, (phase >> stage) & 1u);
+    const int32_t r = ra + i * kR;
+    double v[kR][kK], s[kR];
+#pragma unroll
+    for (int q = 0; q < kR; ++q) {
+      s[q] = 0.0;
+      // a piece ends where a new block of kTriT columns begins: only the last is ragged
+      const T* row = ring + (stage * kR + q) * cap + head(r + q) + t;
+      const bool live = r + q < rb;
+#pragma unroll
+      for (int k = 0; k < kK; ++k)
+        v[q][k] = live && (k + 1 < kK || t + kTriT * k <= r + q) ? static_cast<double>(row[kTriT * k]) : 0.0;
+    }
+#pragma unroll
+    for (int k = 0; k < kK; ++k) {
+      const double wk = sm.ws[t + kTriT * k];
+#pragma unroll
+      for (int q = 0; q < kR; ++q) s[q] = fma(v[q][k], wk, s[q]);
+    }
+    double* red = sm.red + buf * 8 * (kTriT / 32);  // [row][warp]
+    const double sum = warp_reduce_scatter<kR>(s, lane);
+    if (reduce_scatter_writer<kR>(lane)) red[reduce_scatter_index<kR>(lane) * (kTriT / 32) + w] = sum;
+    // every thread has read the stage; the other buffer is written next
+    if (!__syncthreads_and(ok ? 1 : 0)) {
+      if (t == 0)  // the copies still on their way (bounded)
+        for (int j = i; j < min(i + depth, steps); ++j) {
+          const int q = (stage + (j - i)) % depth;
+          tma::mbar_wait(sm.full + q, (phase >> q) & 1u);
+        }
+      return false;
+    }
+    phase ^= 1u << stage;
+    if (t == 0 && i + depth < steps) {
+      tma::fence_proxy_async();
+      fetch(i + depth, stage);
+    }
+    stage = stage + 1 == depth ? 0 : stage + 1;
+    double z = 0.0;
+#pragma unroll
+    for (int j = 0; j < kR / 2; ++j) z += red[(lane & (kR - 1)) * (kTriT / 32) + (lane / kR) * (kR / 2) + j];
+#pragma unroll
+    for (int o = kR; o < 32; o <<= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
+    double zr[kR], wr[kR];
+#pragma unroll
+    for (int q = 0; q < kR; ++q) {
+      zr[q] = __shfl_sync(0xffffffffu, z, q);
+      wr[q] = kInverse ? zr[q] : r + q < rb ? sm.ws[r + q] : 0.0;
+    }
+#pragma unroll
+    for (int k = 0; k < kK; ++k) {
+      const bool edge = !kInverse && k + 1 == kK;  // the block that holds the diagonal
+      double y = v[0][k] * (edge && t + kTriT * k == r ? 0.0 : wr[0]);
+#pragma unroll
+      for (int q = 1; q < kR; ++q) y = fma(v[q][k], edge && t + kTriT * k == r + q ? 0.0 : wr[q], y);
+      acc[k] += y;
+      if (edge) {
+#pragma unroll
+        for (int q = 0; q < kR; ++q)
+          if (t + kTriT * k == r + q) acc[k] += zr[q];
+      }
+    }
+    // L^-T z: the sums of kTriFlush steps are added up with the roundings carried along
+    if (i + 1 == steps || (kInverse && i % kTriFlush == kTriFlush - 1)) {
+#pragma unroll
+      for (int k = 0; k < kK; ++k) {
+        if (t + kTriT * k < rb) {
+          const double2 old = !kInverse || i < kTriFlush ? make_double2(0.0, 0.0) : out[t + kTriT * k];
+          out[t + kTriT * k] = add_carried(old, acc[k]);
+        }
+        acc[k] = 0.0;
+      }
+    }
+  }
+  return true;
+}
+
+template <bool kInverse, class T>
+__global__ void __launch_bounds__(kTriT, 1) k_tri_apply(const TriSeg* __restrict__ seg,
+                                                       const int32_t* __restrict__ cta_seg,
+                                                       const int32_t* __restrict__ dim,
+                                                       const int64_t* __restrict__ m_off, const T* __restrict__ M,
+                                                       const int64_t* __restrict__ v_off,
+                                                       const double* __restrict__ w, double2* __restrict__ slots,
+                                                       int32_t* __restrict__ err) {
+  extern __shared__ __align__(128) double smd[];
+  const TriSmem sm{smd, smd + kTriRing, smd + kTriRing + kTriMaxN,
+                   reinterpret_cast<uint64_t*>(smd + kTriRing + kTriMaxN + kTriRed)};
+  if (threadIdx.x < kTriStages) tma::mbar_init(sm.full + threadIdx.x, 1);
+  tma::fence_mbar_init();
+  const uint64_t pol = evict_first_policy();
+  uint32_t phase = 0;
+  bool ok = true;
+  for (int32_t g = cta_seg[blockIdx.x]; g < cta_seg[blockIdx.x + 1]; ++g) {
+    const TriSeg S = seg[g];
+    double2* out = slots + S.slot;
+    if (ok) {
+      const int32_t n = dim[S.root];
+      const int64_t o = m_off[S.root];
+      const double* wm = w + v_off[S.root];
+      const int kk = (S.rb + kTriT - 1) / kTriT;
+      __syncthreads();  // the piece before still reads ws and the ring
+      for (int32_t i = threadIdx.x; i < kk * kTriT; i += kTriT) sm.ws[i] = i < S.rb ? wm[i] : 0.0;
+      tma::fence_proxy_async();
+      __syncthreads();
+      switch (kk) {
+        case 1: ok = tri_rows<kInverse, 1, 8>(M, o, n, S.ra, S.rb, sm, phase, pol, out); break;
+        case 2: ok = tri_rows<kInverse, 2, 8>(M, o, n, S.ra, S.rb, sm, phase, pol, out); break;
+        case 3: ok = tri_rows<kInverse, 3, 8>(M, o, n, S.ra, S.rb, sm, phase, pol, out); break;
+        case 4: ok = tri_rows<kInverse, 4, 4>(M, o, n, S.ra, S.rb, sm, phase, pol, out); break;
+        case 5: ok = tri_rows<kInverse, 5, 4>(M, o, n, S.ra, S.rb, sm, phase, pol, out); break;
+        case 6: ok = tri_rows<kInverse, 6, 4>(M, o, n, S.ra, S.rb, sm, phase, pol, out); break;
+        case 7: ok = tri_rows<kInverse, 7, 2>(M, o, n, S.ra, S.rb, sm, phase, pol, out); break;
+        default: ok = tri_rows<kInverse, kTriMaxK, 2>(M, o, n, S.ra, S.rb, sm, phase, pol, out); break;
+      }
+    }
+    if (!ok) {
+      if (threadIdx.x == 0) atomicOr(err, kErrWait);
+      for (int32_t i = threadIdx.x; i < S.rb; i += kTriT) out[i] = make_double2(nan(""), 0.0);
+    }
+  }
+}
+
+// y = the sum of every root's slots (pieces root_seg[m] .. root_seg[m + 1], in
+// row order; a piece that ends at row rb holds the columns below rb).
+__global__ void __launch_bounds__(256) k_tri_sum(const TriSeg* __restrict__ seg,
+                                                     const int32_t* __restrict__ root_seg,
+                                                     const int32_t* __restrict__ dim,
+                                                     const int64_t* __restrict__ v_off,
+                                                     const double2* __restrict__ slots, double* __restrict__ y) {
+  const int32_t m = blockIdx.y, c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= dim[m]) return;
+  double2 sum = make_double2(0.0, 0.0);
+  const int32_t g1 = root_seg[m + 1];
+#pragma unroll 4
+  for (int32_t g = root_seg[m]; g < g1; ++g) {
+    const double2 v = c < seg[g].rb ? slots[seg[g].slot + c] : make_double2(0.0, 0.0);
+    sum = add_carried(sum, v.x);
+    sum.y += v.y;
+  }
+  y[v_off[m] + c] = sum.x + sum.y;
+}
+
 // y = S w for symmetric dense blocks S (the roots' S_DD, full column-major
 // storage), reading only the 64 x 64 tiles on and below the diagonal: half
 // the bytes of a full column-dot pass.  k_symv_rows: one CTA per block row
@@ -2369,6 +2586,50 @@ int FetiDP::setup_device() {
     }
     if ((rc = up(&d_pcoff, pcoff)) || (rc = zalloc(&pc_d, std::max<int64_t>(pcoff.back(), 1)))) return rc;
   }
+  // Products that read a triangle once: where the rows are long enough for a
+  // block sum a few rows to cost less than a second read of them.  Roots of 864
+  // unknowns (24^3 in 8: rows of 432 on average) take 28 us for L^-T (L^-1 w) and
+  // 30 for S w here, 25 and 39 with the column-dot and tile passes; roots of 600
+  // (20^3 in 8) 21 and 22 against 10 and 16; 64 roots of 512 (32^3 in 64) 69 and
+  // 78 against 55 and 39.
+  int64_t tri_entries = 0, tri_rows_all = 0;
+  for (int32_t d : rdim) {
+    tri_entries += static_cast<int64_t>(d) * (d + 1) / 2;
+    tri_rows_all += d;
+  }
+  if (max_nD <= kTriMaxN && tri_entries >= kTriMinEntries && tri_entries >= kTriMinRow * tri_rows_all) {
+    // pieces: equal cost a CTA, whole rows, cut where a block of kTriT columns begins
+    int dv = 0, sms = 148;
+    EMG_CK(cudaGetDevice(&dv));
+    EMG_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dv));
+    std::vector<TriSeg> seg;
+    std::vector<int32_t> cta{0}, rseg(rdim.size() + 1, 0);
+    const int64_t total = tri_entries + kTriRowCost * tri_rows_all;
+    int64_t done = 0, slot = 0;
+    double* slots = nullptr;
+    for (size_t q = 0; q < rdim.size(); ++q) {
+      for (int32_t r = 0, ra = 0; r < rdim[q]; ++r) {
+        done += r + 1 + kTriRowCost;
+        const int32_t full = static_cast<int32_t>(cta.size());  // CTAs that end here or before
+        const bool last = static_cast<double>(done) * sms >= static_cast<double>(total) * full;
+        if (!last && r + 1 < rdim[q] && (r + 1) % kTriT != 0) continue;
+        seg.push_back({static_cast<int32_t>(q), ra, r + 1, 0, slot});
+        slot += r + 1;
+        ra = r + 1;
+        if (last) cta.push_back(static_cast<int32_t>(seg.size()));
+      }
+      rseg[q + 1] = static_cast<int32_t>(seg.size());
+    }
+    if (cta.back() < static_cast<int32_t>(seg.size())) cta.push_back(static_cast<int32_t>(seg.size()));
+    EMG_CK(cudaFuncSetAttribute(k_tri_apply<true, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTriSmem));
+    EMG_CK(cudaFuncSetAttribute(k_tri_apply<false, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTriSmem));
+    EMG_CK(cudaFuncSetAttribute(k_tri_apply<false, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTriSmem));
+    tri_ctas = static_cast<int32_t>(cta.size()) - 1;
+    if ((rc = up(&d_tri_seg, seg)) || (rc = up(&d_tri_cta, cta)) || (rc = up(&d_tri_root, rseg)) ||
+        (rc = zalloc(&slots, 2 * slot)))
+      return rc;
+    tri_slots_d = reinterpret_cast<double2*>(slots);
+  }
   // setup solves: n_r x (nP + 1) per subdomain; recovery: one column in union layout
   std::vector<int64_t> roff_s(S), roff1(S);
   std::vector<int32_t> ncol_s(S), ncol1(S, 1);
@@ -2410,11 +2671,11 @@ int FetiDP::setup_device() {
       (rc = zalloc(&xacc_d, P.n_dofs)) || (rc = zalloc(&rglob_d, P.n_dofs)) ||
       (rc = zalloc(&root_tmp_d, nd * max_ncol)) || (rc = zalloc(&rold_d, nl)) || (rc = zalloc(&zm_d, nl)))
     return rc;
-  if ((rc = zallocf(&S32_d, P.root_off[S])) || (rc = zallocf(&fDa32_d, fsz)) || (rc = zallocf(&fDb32_d, fsz)) ||
+  if ((rc = zallocf(&S32_d, P.root_off[S] + kTriPad)) || (rc = zallocf(&fDa32_d, fsz)) || (rc = zallocf(&fDb32_d, fsz)) ||
       (rc = zallocf(&fDaT32_d, fsz)) || (rc = zallocf(&fDbT32_d, fsz)))
     return rc;
   if ((rc = zalloc(&fac_d, P.fac_size + nc2 + fsz)) || (rc = zalloc(&upd_d, P.upd_pool)) ||
-      (rc = zalloc(&S_d, P.root_off[S])) || (rc = zalloc(&Linv_d, P.root_off[S])) ||
+      (rc = zalloc(&S_d, P.root_off[S] + kTriPad)) || (rc = zalloc(&Linv_d, P.root_off[S] + kTriPad)) ||
       (rc = zalloc(&Lcc_d, nc * nc)) || (rc = zalloc(&phi_d, phi_size)) || (rc = zalloc(&vs_d, vs_size)) ||
       (rc = zalloc(&v1_d, P.vec_rows)) || (rc = zalloc(&cblk_d, P.cblk_off[S])) ||
       (rc = zalloc(&h_d, P.pri_off[S])) || (rc = zalloc(&gc_d, nc)) || (rc = zalloc(&uc_d, nc)) ||
@@ -2703,9 +2964,19 @@ void FetiDP::coarse_apply_t(const RhsDev& R, const double* w, const double* add,
   k_coarse_sum<<<blocks_for(plan.n_coarse, 128), 128, 0, st>>>(plan.n_coarse, d_coarse_ptr, cdots_d, add, t);
 }
 
-// y = S_DD w for every root, the lower tiles only (k_symv_rows, k_symv_cols).
+// y = L^-T (L^-1 w) or S w of every root, each triangle read once.
+template <bool kInverse, class T>
+void FetiDP::tri_apply(const T* M, const double* w, double* y) {
+  k_tri_apply<kInverse, T><<<tri_ctas, kTriT, kTriSmem, st>>>(d_tri_seg, d_tri_cta, d_rdim, d_roff, M, d_rvoff, w,
+                                                             tri_slots_d, err_d);
+  k_tri_sum<<<dim3(blocks_for(max_nD, 256), static_cast<unsigned>(n_roots)), 256, 0, st>>>(
+      d_tri_seg, d_tri_root, d_rdim, d_rvoff, tri_slots_d, y);
+}
+
+// y = S_DD w for every root, half of each block read (symv_roots).
 template <class T>
 void FetiDP::symv_roots(const T* M, const double* w, double* y) {
+  if (tri_ctas > 0) { tri_apply<false>(M, w, y); return; }
   const unsigned nb = static_cast<unsigned>((max_nD + kSy - 1) / kSy);
   k_symv_rows<T><<<dim3(nb, static_cast<unsigned>(n_roots)), 256, 0, st>>>(n_roots, d_rdim, d_roff, M, d_rvoff,
                                                                            d_pcoff, w, y, pc_d);
@@ -2729,9 +3000,13 @@ void FetiDP::apply_F(const double* p, double* q, double* part) {
   const int64_t ne = P.dual_off[P.n_parts];
   RhsDev R{phi_d, d_roff_s, d_ncol_s, d_voff_s, vs_d};
   k_dual_gather<<<blocks_for(ne, 256), 256, 0, st>>>(ne, d_dual_lam, d_dual_sign, nullptr, p, w_d);
-  const dim3 gr(static_cast<unsigned>((max_nD + gemv_warps - 1) / gemv_warps), static_cast<unsigned>(n_roots));
-  k_block_colgemv<double><<<gr, 32 * gemv_warps, 0, st>>>(n_roots, d_rdim, d_roff, Linv_d, d_rvoff, w_d, y2_d, 0);
-  k_block_colgemv<double><<<gr, 32 * gemv_warps, 0, st>>>(n_roots, d_rdim, d_roff, Linv_d, d_rvoff, y2_d, y_d, 1);
+  if (tri_ctas > 0) {
+    tri_apply<true>(Linv_d, w_d, y_d);
+  } else {
+    const dim3 gr(static_cast<unsigned>((max_nD + gemv_warps - 1) / gemv_warps), static_cast<unsigned>(n_roots));
+    k_block_colgemv<double><<<gr, 32 * gemv_warps, 0, st>>>(n_roots, d_rdim, d_roff, Linv_d, d_rvoff, w_d, y2_d, 0);
+    k_block_colgemv<double><<<gr, 32 * gemv_warps, 0, st>>>(n_roots, d_rdim, d_roff, Linv_d, d_rvoff, y2_d, y_d, 1);
+  }
   if (P.n_coarse > 0) {
     coarse_apply_t(R, w_d, nullptr, t_d);
     coarse_solve(t_d, uc_d);

@@ -52,6 +52,13 @@ struct FacesDev {
   const int64_t* fac;  // offset of the face's Sa + Sb factor block in fac
 };
 
+// Rows [ra, rb) of a root's triangle that one CTA handles, and where its part of
+// the product goes.
+struct TriSeg {
+  int32_t root, ra, rb, pad;
+  int64_t slot;
+};
+
 struct FetiStats {
   int32_t iterations = 0;         // multiplier iterations over all correction passes
   int32_t refinements = 0;        // FETI-DP passes (1 + defect corrections)
@@ -101,6 +108,10 @@ struct FetiDP {
   int64_t *d_rfac = nullptr, *d_roff = nullptr, *d_rvoff = nullptr;
   int64_t* d_pcoff = nullptr;  // per root: offset of its column-sum slots in pc_d
   double* pc_d = nullptr;       // column sums of the tiles below the diagonal (symmetric S_DD products)
+  TriSeg* d_tri_seg = nullptr;  // pieces of the products that read a triangle once
+  int32_t *d_tri_cta = nullptr, *d_tri_root = nullptr;  // first piece of every CTA, of every root
+  double2* tri_slots_d = nullptr;  // every piece's part: (sum, carried roundings)
+  int32_t tri_ctas = 0;  // 0: the column-dot and tile passes
   int32_t* d_cdim = nullptr;
   int64_t *d_cfac = nullptr, *d_czero = nullptr;
   int64_t coarse_fac = 0;
@@ -182,6 +193,8 @@ struct FetiDP {
   void coarse_apply_t(const RhsDev& R, const double* w, const double* add, double* t);
   template <class T>
   void symv_roots(const T* M, const double* w, double* y);
+  template <bool kInverse, class T>
+  void tri_apply(const T* M, const double* w, double* y);
   void apply_F(const double* p, double* q, double* part);
   void apply_M(const double* r, double* z, double* part);
   int dot(const double* a, const double* b, int64_t n, int which);
