@@ -1758,7 +1758,7 @@ void setup_resident(KrylovWorkspace& w) {
   }
   const int64_t ns = (w.n + kSliceRows - 1) / kSliceRows;
   const int64_t g = std::min<int64_t>(std::min(sms, kResMaxGrid), (ns + kResMinSlices - 1) / kResMinSlices);
-  if (!coop || g < 1 || 3 * kResVals * g > 4 * w.grid) return;
+  if (!coop || g < 1 || kResBuffers * kResVals * g > 4 * w.grid) return;
   const ResidentShape* shape = nullptr;
   for (const ResidentShape& h : kResShapes)
     if (!shape && (ns + g - 1) / g <= h.rows * (h.threads / 32)) shape = &h;
@@ -1792,7 +1792,7 @@ bool launch_resident(DevCsr& A, const double* b, double* x, int32_t precond, boo
   const ResidentArgs args{S, b, x, A.row_ptr, A.col, A.val, precond,
                           reinterpret_cast<double2*>(w.zp), w.z, w.p, reinterpret_cast<unsigned long long*>(w.partial),
                           w.state, w.hist, w.hist_cap, stage};
-  if (cudaMemsetAsync(w.partial, 0xff, sizeof(double) * 3 * kResVals * w.res_grid, st) != cudaSuccess) return false;
+  if (cudaMemsetAsync(w.partial, 0xff, sizeof(double) * kResBuffers * kResVals * w.res_grid, st) != cudaSuccess) return false;
   cudaLaunchConfig_t c = {};
   c.gridDim = dim3(static_cast<unsigned>(w.res_grid));
   c.blockDim = dim3(static_cast<unsigned>(kResShapes[w.res_shape].threads));

@@ -24,6 +24,7 @@ namespace emg {
 namespace {
 
 constexpr int kResVals = 2;      // values of one reduction at most
+constexpr int kResBuffers = 5;   // reductions before a slot is used again (GridSums)
 constexpr int kResMaxGrid = 256; // a thread polls one block's slots
 constexpr unsigned long long kResEmpty = ~0ull;  // an unpublished slot (a NaN no sum produces)
 
@@ -36,7 +37,7 @@ struct ResidentArgs {
   int32_t precond;
   double2* zp;                // CG: (z, old p) of every row; what other blocks gather, permuted numbering
   double *z, *p;              // BiCGSTAB: z and p, likewise
-  unsigned long long* slots;  // 3 x grid x kResVals, all kResEmpty at launch
+  unsigned long long* slots;  // kResBuffers x grid x kResVals, all kResEmpty at launch
   SolverState* st;
   double* hist;
   int32_t hist_cap;
@@ -47,9 +48,12 @@ struct ResidentArgs {
 // same totals.  kFence: also the barrier that makes the blocks' earlier writes
 // to global memory visible to each other (the block's slot is published with
 // release semantics after its barrier).  Without it a block's sums still depend on
-// all it has read, so what it read may be overwritten afterwards.  Three slot
-// buffers in turn: when a block resets its slots of the buffer after this one,
-// every block has read them (it has published to the buffer in between).
+// all it has read, so what it read may be overwritten afterwards.  Five slot
+// buffers in turn: reduction k resets the block's slots of reduction k + 3.
+// Every block has read what they held, the sums of k - 2, since it has
+// published to k - 1; and the reset is seen before anything is polled there,
+// since one of the reductions k .. k + 2 carries the fence in every sequence
+// the kernels run (CG alternates, BiCGSTAB has two without in a row at most).
 // False when a wait ran out.
 template <int T>
 struct GridSums {
@@ -71,8 +75,8 @@ struct GridSums {
       if (lane == 0) part[i][w] = s;
     }
     __syncthreads();
-    unsigned long long* now = slots + static_cast<int64_t>(k % 3) * (kResVals * G);
-    unsigned long long* next = slots + static_cast<int64_t>((k + 1) % 3) * (kResVals * G);
+    unsigned long long* now = slots + static_cast<int64_t>(k % kResBuffers) * (kResVals * G);
+    unsigned long long* next = slots + static_cast<int64_t>((k + 3) % kResBuffers) * (kResVals * G);
     if (w < K) {
       const double s = warp_sum(lane < T / 32 ? part[w][lane] : 0.0);
       if (lane == 0) {
