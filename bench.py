@@ -739,13 +739,13 @@ def fetidp_variants(fd, names, steps, warmup, stream, dev):
             res[name] = {"what": what, "failed": failed}
             continue
         its = max(int(st["iterations"]), 1)
-        # dense blocks read per multiplier iteration: L^-1 (lower part, then
-        # the stored transpose: the whole n_D^2 block once), the S_DD tiles on
-        # and below the diagonal and the four deluxe blocks of every face
-        # (FP32 copies of both with the FP32 preconditioner)
+        # what a multiplier iteration cannot do without: L^-1's triangle once
+        # (n_D (n_D + 1) / 2; small roots read it a second time, transposed), the
+        # S_DD tiles on and below the diagonal and the four deluxe blocks of
+        # every face (FP32 copies of both with the FP32 preconditioner)
         fi = fd.info()
         pw = 4 if precond == 3 else 8
-        nb = fi["dual_block_doubles"] * 8 + fi["sym_tile_doubles"] * pw + 4 * fi["face_block_doubles"] * pw
+        nb = (fi["dual_block_doubles"] + fi["sum_nD"]) * 4 + fi["sym_tile_doubles"] * pw + 4 * fi["face_block_doubles"] * pw
         peak, _ = measured_peak()
         per_it = st["lambda_ms"] / its
         res[name] = {"what": what, "ms": statistics.mean(per), "ms_steps": [round(v, 3) for v in per],
