@@ -253,6 +253,8 @@ __global__ void __launch_bounds__(kIlThreads) k_ilu_upper(const int32_t* __restr
 // memory (which is which is known when the rows are laid out).
 constexpr int kIlWarps = 16;
 constexpr int kIlRing = 12288;  // values (96 KB; a multiple of 32)
+constexpr int kIlZero = kIlRing;  // a slot behind the ring that stays 0: what padding entries read
+constexpr int kIlRingSize = kIlRing + 2;
 constexpr int kIlGroups = 2;  // groups of four entries of a row held in registers; the rest are loaded when used
 
 struct IlSweep {
@@ -262,7 +264,8 @@ struct IlSweep {
   int32_t* off = nullptr;   // nchunk + 1: first entry group of every chunk
   int32_t* in = nullptr;    // 32 nchunk: index of the row's right-hand side, -1 = padding
   int32_t* row = nullptr;   // 32 nchunk: matrix row, -1 = padding
-  int4* pos = nullptr;      // [group][lane]: four entries' columns: the ring slot, or ~position once it has left the ring
+  int4* pos = nullptr;      // [group][lane]: four entries' columns: the ring slot, or ~position once it has left the
+                            // ring; padding: kIlZero
   int32_t* src = nullptr;   // [group][lane][4]: their index in the factor, -1 = padding
   double2* val = nullptr;   // [group][2][lane]: their values, refreshed with every factorization
   double* dinv = nullptr;   // 32 nchunk: 1 / u_ii (null: unit diagonal)
@@ -302,7 +305,7 @@ __device__ __forceinline__ void il_sweep(const IlSweep& S, const double* in, dou
         load(off + g, pp + 4 * g, pv + 4 * g);
       } else {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) { pp[4 * g + j] = lane; pv[4 * g + j] = 0.0; }
+        for (int j = 0; j < 4; ++j) { pp[4 * g + j] = kIlZero; pv[4 * g + j] = 0.0; }
       }
     }
     rhs = idx1 >= 0 ? in[idx1] : 0.0;
@@ -361,7 +364,7 @@ __device__ __forceinline__ void il_sweep(const IlSweep& S, const double* in, dou
 // against 1.86 (the one SM's bandwidth, about 55 GB/s here, is what bounds it).
 constexpr int64_t kIlMaxRows = 1000;
 constexpr int kIlMaxLevels = 8000;  // of a sweep: the level offsets of both lie beside the ring
-size_t ilu_sweep_smem(int32_t nl, int32_t nu) { return sizeof(double) * kIlRing + sizeof(int32_t) * (nl + nu + 2); }
+size_t ilu_sweep_smem(int32_t nl, int32_t nu) { return sizeof(double) * kIlRingSize + sizeof(int32_t) * (nl + nu + 2); }
 
 // z = U^-1 L^-1 r
 __global__ void __launch_bounds__(32 * kIlWarps) k_ilu_sweeps(IlSweep L, IlSweep U, const double* r, double* ypos,
@@ -369,8 +372,8 @@ __global__ void __launch_bounds__(32 * kIlWarps) k_ilu_sweeps(IlSweep L, IlSweep
                                                               const IlState* __restrict__ st) {
   extern __shared__ __align__(16) double il_ring[];
   if (st->done) return;
-  int32_t* lev = reinterpret_cast<int32_t*>(il_ring + kIlRing);  // both sweeps' level offsets
-  for (int i = threadIdx.x; i < kIlRing; i += blockDim.x) il_ring[i] = 0.0;
+  int32_t* lev = reinterpret_cast<int32_t*>(il_ring + kIlRingSize);  // both sweeps' level offsets
+  for (int i = threadIdx.x; i < kIlRingSize; i += blockDim.x) il_ring[i] = 0.0;
   for (int i = threadIdx.x; i <= L.nlev; i += blockDim.x) lev[i] = L.lev[i];
   for (int i = threadIdx.x; i <= U.nlev; i += blockDim.x) lev[L.nlev + 1 + i] = U.lev[i];
   __syncthreads();
@@ -642,9 +645,13 @@ int ilu_sweeps(IluState& s, const std::vector<int32_t>& rp, const std::vector<in
         const int32_t b = i < 0 ? 0 : up ? diag[i] + 1 : rp[i], e = i < 0 ? 0 : up ? rp[i + 1] : diag[i];
         for (int32_t j = 0; j < 4 * len; ++j) {
           const size_t k = base + 128 * static_cast<size_t>(j / 4) + 4 * q + j % 4;
-          const int32_t p = b + j < e ? at[col[b + j]] : 32 * c + q;
+          if (b + j >= e) {
+            pos[k] = kIlZero;
+            continue;
+          }
+          const int32_t p = at[col[b + j]];
           pos[k] = p >= 32 * level_end[c] - kIlRing ? p % kIlRing : ~p;
-          src[k] = b + j < e ? b + j : -1;
+          src[k] = b + j;
         }
       }
       off.push_back(static_cast<int32_t>(pos.size() / 128));
