@@ -179,9 +179,9 @@ constexpr double kPivRel = 1e-11;
 // serial chain, one CTA's latency per panel of every front, so the layout is
 // chosen for the chain: one warp holds the sub-panel's columns in
 // registers (a lane two rows), no barrier between columns, and the next
-// pivot a'_cc - a'_c^2 / v is formed from unscaled entries fetched while the
-// root of this one is on its way, so a column costs a reciprocal root and two
-// operations; all eight warps subtract the
+// pivot a'_cc - (a'_c / sqrt v)^2 is formed from unscaled entries fetched while
+// the root of this one is on its way, so a column costs a reciprocal root and
+// two operations; all eight warps subtract the
 // rank-kPW product from the columns to its right (8 x 8 tiles on the FP64
 // tensor cores), two barriers a sub-panel.  Pivot test against d0, the
 // matrix's own diagonal, when given.  Then X = L^-1: the four 16 x 16
@@ -274,7 +274,10 @@ __device__ __forceinline__ void potrf_panel(double* __restrict__ A, int32_t fs, 
         a0[c] *= ri;
         a1[c] *= ri;
         if (lane == 0) sm.rinv[c0 + c] = ri;
-        if (c + 1 < kPW) v = fma(-(p1 * p1), ri * ri, pp);
+        if (c + 1 < kPW) {  // scaled before it is squared: p1 * p1 can leave the range
+          const double l = p1 * ri;
+          v = fma(-l, l, pp);
+        }
 #pragma unroll
         for (int q = c + 1; q < kPW; ++q) {
           const double m = __shfl_sync(0xffffffffu, a0[c], (c0 + q) & 31);
