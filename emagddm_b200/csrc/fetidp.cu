@@ -207,18 +207,6 @@ __device__ __forceinline__ void dmma_8x8x4(double (&d)[2], double a, double b) {
                : "d"(a), "d"(b));
 }
 
-// 1 / sqrt(v) to within an ulp, without the branches of the library's (which
-// keep the columns' chains from overlapping): the hardware's approximation
-// y (22 bits) and one step of third order, y (1 + e / 2 + 3 e^2 / 8) with
-// e = 1 - v y^2.  Denormal pivots take the library's.
-__device__ __forceinline__ double inv_sqrt(double v) {
-  if (__double2hiint(v) < 0x00100000) return rsqrt(v);
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(v));
-  const double e = fma(-(v * y), y, 1.0);
-  return fma(y * e, fma(0.375, e, 0.5), y);
-}
-
 __device__ __forceinline__ void potrf_panel(double* __restrict__ A, int32_t fs, int32_t nb,
                                             const double* __restrict__ d0, int32_t* __restrict__ err,
                                             PotrfSmem& sm) {
@@ -268,7 +256,7 @@ __device__ __forceinline__ void potrf_panel(double* __restrict__ A, int32_t fs, 
         }
         const bool bad = !(v > 0.0) || !(v > least[c]);
         fail |= bad;  // a unit pivot keeps the rest finite; the factorization is reported as failed
-        const double root = inv_sqrt(v), ri = bad ? 1.0 : root;
+        const double root = rsqrt(v), ri = bad ? 1.0 : root;
         v = bad ? 1.0 : v;
         if (lane == ((c0 + c) & 31)) a0[c] = v;
         a0[c] *= ri;
