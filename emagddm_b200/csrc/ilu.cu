@@ -363,6 +363,11 @@ __device__ __forceinline__ void il_sweep(const IlSweep& S, const double* in, dou
 // level on average: 507 (32^3) 333 ms a solve against 593, 1,144 (48^3) 1.97 s
 // against 1.86 (the one SM's bandwidth, about 55 GB/s here, is what bounds it).
 constexpr int64_t kIlMaxRows = 1000;
+// And, since the groups past those in registers are loaded one after another, at
+// this many of them in a level's longest row on average. A level of band matrices
+// with 8 / 12 / 20 / 24 / 28 / 100 entries a row takes 0.26 / 0.67 / 1.9 / 3.3 /
+// 4.2 / 23.6 us here and 3.1 to 3.6 us as a launch.
+constexpr int64_t kIlMaxTail = 4;
 constexpr int kIlMaxLevels = 8000;  // of a sweep: the level offsets of both lie beside the ring
 size_t ilu_sweep_smem(int32_t nl, int32_t nu) { return sizeof(double) * kIlRingSize + sizeof(int32_t) * (nl + nu + 2); }
 
@@ -603,15 +608,28 @@ int ilu_sweeps(IluState& s, const std::vector<int32_t>& rp, const std::vector<in
   if (n > kIlMaxRows * static_cast<int64_t>(s.lptr.size() - 1) ||
       std::max(s.lptr.size(), s.uptr.size()) > static_cast<size_t>(kIlMaxLevels))
     return EMG_SUCCESS;
+  bool up = false;
+  auto count = [&](int32_t i) { return up ? rp[i + 1] - diag[i] - 1 : diag[i] - rp[i]; };
+  for (bool u : {false, true}) {
+    up = u;
+    const std::vector<int32_t>&ptr = up ? s.uptr : s.lptr, &rows = up ? urows : lrows;
+    int64_t tail = 0;
+    for (size_t l = 0; l + 1 < ptr.size(); ++l) {
+      int32_t longest = 0;
+      for (int32_t k = ptr[l]; k < ptr[l + 1]; ++k) longest = std::max(longest, count(rows[k]));
+      tail += std::max((longest + 3) / 4 - kIlGroups, 0);
+    }
+    if (tail > kIlMaxTail * static_cast<int64_t>(ptr.size() - 1)) return EMG_SUCCESS;
+  }
   std::vector<int32_t> lpos(n);
   int rc = EMG_SUCCESS;
-  for (int up = 0; up < 2; ++up) {
+  for (bool u : {false, true}) {
+    up = u;
     const std::vector<int32_t>& ptr = up ? s.uptr : s.lptr;
     std::vector<int32_t>& rows = up ? urows : lrows;
     IlSweep& S = up ? s.usw : s.lsw;
     std::vector<int32_t> at(n), lev(1, 0), off(1, 0), in, row, pos, src;
     S.nlev = static_cast<int32_t>(ptr.size()) - 1;
-    auto count = [&](int32_t i) { return up ? rp[i + 1] - diag[i] - 1 : diag[i] - rp[i]; };
     for (int32_t l = 0; l < S.nlev; ++l) {  // a level's longest rows first: chunks of even rows
       std::stable_sort(rows.begin() + ptr[l], rows.begin() + ptr[l + 1],
                        [&](int32_t a, int32_t b) { return count(a) > count(b); });
