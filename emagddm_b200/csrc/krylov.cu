@@ -631,9 +631,9 @@ __device__ __forceinline__ bool reduce_partials(const double (&vals)[kVals], dou
 }
 
 // ------------------------------------------------------------ SELL build ----
-// Warp per slice: column index (permuted), CSR source and, for products in the
-// matrix's own numbering (ocol not null), own column of every slot; rows at or
-// past n are all padding.
+// Warp per slice: column index (permuted), own column (for products in the
+// matrix's own numbering) and CSR source of every slot; rows at or past n are
+// all padding.
 __global__ void k_sell_fill(int64_t n, int64_t nslices, const int64_t* __restrict__ sp,
                             const int32_t* __restrict__ perm, const int32_t* __restrict__ iperm,
                             const int32_t* __restrict__ rp, const int32_t* __restrict__ ccol,
@@ -655,7 +655,7 @@ __global__ void k_sell_fill(int64_t n, int64_t nslices, const int64_t* __restric
     for (int j = 0; j < len; ++j) {
       const int64_t k = b0 + static_cast<int64_t>(kGroupStride) * j + lane;
       const int64_t kc = EMG_SELL_PACKED ? packed_col_index(k) : k;
-      if (ocol) ocol[k] = j < rl ? ccol[a + j] : 0;
+      ocol[k] = j < rl ? ccol[a + j] : 0;
       if (j < rl) {
         col[kc] = iperm[ccol[a + j]];
         src[k] = a + j;
@@ -813,12 +813,6 @@ __global__ void __launch_bounds__(kThreads) k_product(Sell A, const int32_t* __r
                                                       const double* __restrict__ x, double* __restrict__ y) {
   A.col = A.ocol;
   sell_rows<false>(A, x, [&](int64_t row, double s) { y[perm[row]] = s; });
-}
-
-__global__ void k_sell_own_columns(int64_t slots, const int32_t* __restrict__ src, const int32_t* __restrict__ ccol,
-                                   int32_t* __restrict__ ocol) {
-  // padding multiplies column 0 by 0, as the masked entries past a row's end do
-  for (int64_t i = gtid(); i < slots; i += gstride()) ocol[i] = src[i] >= 0 ? ccol[src[i]] : 0;
 }
 
 template <int kMode>
@@ -1407,7 +1401,7 @@ int grid_size() {
 
 // Host: permutation sorting rows by length inside windows (stable), slice
 // offsets; device: slots.
-int build_sell(DevCsr& A, bool own_columns, cudaStream_t st) {
+int build_sell(DevCsr& A, cudaStream_t st) {
   if (!A.sell) A.sell = new Sell();
   Sell& S = *A.sell;
   const int64_t n = A.n;
@@ -1443,7 +1437,7 @@ int build_sell(DevCsr& A, bool own_columns, cudaStream_t st) {
   const size_t ns = static_cast<size_t>(std::max<int64_t>(S.slots, 1));
   EMG_CK(cudaMallocAsync(&iperm, sizeof(int32_t) * n, st));
   EMG_CK(cudaMallocAsync(&S.src, sizeof(int32_t) * ns, st));
-  if (own_columns) EMG_CK(cudaMallocAsync(&S.ocol, sizeof(int32_t) * ns, st));
+  EMG_CK(cudaMallocAsync(&S.ocol, sizeof(int32_t) * ns, st));
   if (EMG_SELL_PACKED) {  // one buffer: 32-slot chunks of values then columns
     EMG_CK(cudaMallocAsync(&S.val, (sizeof(double) + sizeof(int32_t)) * ns, st));
     S.col = reinterpret_cast<int32_t*>(S.val);
@@ -1544,11 +1538,10 @@ int build_sell(DevCsr& A, bool own_columns, cudaStream_t st) {
 
 void tune_sell_grid(DevCsr& A, cudaStream_t st);
 
-// own_columns: products in the matrix's own numbering (csr_spmv) will be asked for
-int ensure_sell(DevCsr& A, cudaStream_t st, bool own_columns = false) {
+int ensure_sell(DevCsr& A, cudaStream_t st) {
   bool fresh = false;
   if (!A.sell) {
-    int rc = build_sell(A, own_columns, st);
+    int rc = build_sell(A, st);
     if (rc) return rc;
     fresh = true;
   }
@@ -2090,13 +2083,9 @@ int csr_spmv(DevCsr& A, const double* x, double* y, cudaStream_t st) {
   if (!x || !y) { set_error("null vector"); return EMG_INVALID_INPUT; }
   int rc = ensure_ws(A, false, 1, st);
   if (rc) return rc;
-  rc = ensure_sell(A, st, true);
+  rc = ensure_sell(A, st);
   if (rc) return rc;
-  Sell& S = *A.sell;
-  if (!S.ocol && S.slots > 0) {  // built by a solver
-    EMG_CK(cudaMallocAsync(&S.ocol, sizeof(int32_t) * S.slots, st));
-    k_sell_own_columns<<<grid_size(), kThreads, 0, st>>>(S.slots, S.src, A.col, S.ocol);
-  }
+  const Sell& S = *A.sell;
   const int64_t warps = std::max<int64_t>(S.nslices, 1);
   const int grid = static_cast<int>(std::min<int64_t>(sell_grid<k_product>(S, grid_size()),
                                                       (warps + kThreads / 32 - 1) / (kThreads / 32)));
