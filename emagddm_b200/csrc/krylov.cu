@@ -3,12 +3,10 @@
 // 343-503 and :869-1118), with the same iteration, stopping and failure rules.
 //
 // Matrix format inside the solvers: SELL-32-sigma.  Rows are sorted by length
-// (descending) inside windows of 4096 rows and cut into slices of 32 rows; the
-// 8 slices of a 256-row group are padded to the group's longest row and
-// stored entry-interleaved (entry j of the 8 slices is one 2 KB run of
-// values), so one warp reads a slice with 256-byte coalesced loads, every lane
-// has a whole row (no shuffles, many independent loads in flight), and the 8
-// warps of a block stream one contiguous run together.  The solvers run in the
+// (descending) inside windows of 4096 rows and cut into slices of 32 rows,
+// padded to the slice's longest row and stored entry by entry, so one warp
+// reads a slice with 256-byte coalesced loads and every lane has a whole row
+// (no shuffles, many independent loads in flight).  The solvers run in the
 // permuted numbering (P A P^T, P b): all vector kernels stay contiguous; b is
 // permuted on entry and x on exit.  The CSR handed in stays the exported form.
 //
@@ -60,10 +58,9 @@ struct SolverState {
   uint32_t gen;        // grid-barrier generation of the fused CG update
 };
 
-// SELL-32-sigma copy of a DevCsr in the permuted numbering, slices in
-// interleaved groups of kGroup.
+// SELL-32-sigma copy of a DevCsr in the permuted numbering.
 struct Sell {
-  int64_t n = 0, nslices = 0, ngroups = 0, slots = 0;
+  int64_t n = 0, nslices = 0, slots = 0;
   int64_t max_tile_slots = 0;    // largest 8-slice tile (bulk-copy stage size)
   bool tma = false;              // stages of the bulk-copy kernels fit in shared memory
   bool ws = false;               // warp-specialized bulk-copy SpMV in use
@@ -71,9 +68,7 @@ struct Sell {
   int ws_grid = 0;
   size_t ws_smem = 0;
   int32_t* perm = nullptr;       // new row -> old row
-  int64_t* slice_ptr = nullptr;  // ngroups + 1 slot offsets of the slice groups (multiples of 32 kGroup)
-  int16_t* dcol = nullptr;       // column - row of every slot, when all fit in 16 bits
-  bool narrow = false;           // dcol in use (col freed): 10 bytes per slot instead of 12
+  int64_t* slice_ptr = nullptr;  // nslices + 1 slot offsets of the slices (multiples of 32)
   int32_t* col = nullptr;        // permuted column of every slot
   int32_t* src = nullptr;        // CSR index of every slot, -1 = padding
   int32_t* ocol = nullptr;       // column of every slot in the matrix's own numbering (products, csr_spmv)
@@ -149,12 +144,6 @@ __device__ __forceinline__ int64_t gstride() {
 #ifndef EMG_SELL_WS_STAGES
 #define EMG_SELL_WS_STAGES 2
 #endif
-// 16-bit column offsets (10 instead of 12 bytes per slot) when the matrix
-// bandwidth allows: fewer bytes, but measured slower than 32-bit columns on
-// B200 for the 64^3 curl-curl matrix, so off by default.
-#ifndef EMG_SELL_NARROW
-#define EMG_SELL_NARROW 0
-#endif
 #ifndef EMG_SELL_UNROLL
 #define EMG_SELL_UNROLL 4  // row entries per batch of loads in the plain SELL loop
 #endif
@@ -170,41 +159,19 @@ __device__ __forceinline__ int64_t gstride() {
 #ifndef EMG_SELL_BATCH
 #define EMG_SELL_BATCH 8
 #endif
-// Slices per group: the kGroup slices of a group share one length and are
-// interleaved entry by entry (slot of entry j, slice w, lane l at
-// group_base + 32 kGroup j + 32 w + l), so the kGroup warps of a block that
-// work on one group read one contiguous 32 kGroup-slot run per entry.
-#ifndef EMG_SELL_GROUP
-#define EMG_SELL_GROUP 1
-#endif
 // Slice order over the warps: 0 = the warps of a block take adjacent slices
 // (slice = global warp id + k * warps); 1 = they take slices gridDim.x apart,
 // which spreads the concurrent streams of an SM over memory (64.1 vs 65.6 us
-// for the 64^3 CG matrix on B200; interleaving the slices of a block instead,
-// EMG_SELL_GROUP=8, was slower: 75.5 us).
+// for the 64^3 CG matrix on B200; interleaving the slices of a block instead was
+// slower: 75.5 us).
 #ifndef EMG_SELL_SPREAD
 #define EMG_SELL_SPREAD 1
 #endif
-constexpr int kGroup = EMG_SELL_GROUP;
-constexpr int kGroupStride = 32 * kGroup;
 
-// Packed slots: every 32-slot chunk (one warp's entry) is stored as 256 B of
-// values followed by 128 B of columns, one stream per warp instead of two.
-#ifndef EMG_SELL_PACKED
-#define EMG_SELL_PACKED 0
-#endif
-constexpr int kChunkBytes = 384;
-__host__ __device__ __forceinline__ int64_t packed_val_index(int64_t k) { return (k >> 5) * (kChunkBytes / 8) + (k & 31); }
-__host__ __device__ __forceinline__ int64_t packed_col_index(int64_t k) {
-  return (k >> 5) * (kChunkBytes / 4) + 64 + (k & 31);
-}
-
-// Base slot (entry 0, lane 0) and entry count of slice s.
-__device__ __forceinline__ void slice_span(const int64_t* __restrict__ gp, int64_t s, int64_t& base, int& len) {
-  const int64_t g = s / kGroup;
-  const int64_t b0 = gp[g];
-  len = static_cast<int>((gp[g + 1] - b0) / kGroupStride);
-  base = b0 + 32 * (s - g * kGroup);
+// First slot and entry count of slice s.
+__device__ __forceinline__ void slice_span(const int64_t* __restrict__ sp, int64_t s, int64_t& base, int& len) {
+  base = sp[s];
+  len = static_cast<int>((sp[s + 1] - base) / kSliceRows);
 }
 
 // Warp per slice, lane per row, as one software pipeline over all slices of
@@ -215,9 +182,8 @@ __device__ __forceinline__ void slice_span(const int64_t* __restrict__ gp, int64
 // with an exposed load.  A slice without entries takes one batch of masked
 // loads; entries past a row's length are masked (value 0, column 0) and add
 // +0 after the real ones, so every row is summed in CSR order.  Calls
-// out(row, y_row) for every real row.  Unpacked slots; kNarrow: columns as
-// 16-bit offsets from the row (A.dcol).
-template <bool kNarrow, class Out>
+// out(row, y_row) for every real row.
+template <class Out>
 __device__ __forceinline__ void sell_rows_stream(const Sell& A, const double* __restrict__ x, Out out) {
   const int lane = threadIdx.x & 31;
   const int64_t nwarps = gstride() >> 5;
@@ -226,7 +192,6 @@ __device__ __forceinline__ void sell_rows_stream(const Sell& A, const double* __
   const uint64_t pol = evict_first_policy();
   const int64_t* __restrict__ sp = A.slice_ptr;
   const int32_t* __restrict__ col = A.col;
-  const int16_t* __restrict__ dcol = A.dcol;
   const double* __restrict__ val = A.val;
   constexpr int U = EMG_SELL_BATCH;
 #if EMG_SELL_SPREAD == 2
@@ -256,11 +221,9 @@ __device__ __forceinline__ void sell_rows_stream(const Sell& A, const double* __
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const bool in = fj + u < flen;
-      const int64_t k = fbase + static_cast<int64_t>(kGroupStride) * (fj + u);
-      if constexpr (kNarrow) c[u] = in ? static_cast<int>(fs * kSliceRows + lane) + ld_stream(dcol + k, pol) : 0;
-      else if constexpr (EMG_SELL_PACKED) c[u] = in ? ld_stream(col + packed_col_index(k), pol) : 0;
-      else c[u] = in ? ld_stream(col + k, pol) : 0;
-      v[u] = in ? ld_stream(val + (EMG_SELL_PACKED ? packed_val_index(k) : k), pol) : 0.0;
+      const int64_t k = fbase + static_cast<int64_t>(kSliceRows) * (fj + u);
+      c[u] = in ? ld_stream(col + k, pol) : 0;
+      v[u] = in ? ld_stream(val + k, pol) : 0.0;
     }
     fj += U;
     last = fj >= flen;
@@ -303,8 +266,7 @@ __device__ __forceinline__ void sell_rows_stream(const Sell& A, const double* __
 // out(row, y_row) for every real row.  Entries of a row are summed in CSR
 // order, EMG_SELL_UNROLL loads in flight per lane at a time (with
 // EMG_SELL_PIPE=1 the next batch of the same slice as well).
-// kNarrow: columns are stored as 16-bit offsets from the row (A.dcol).
-template <bool kNarrow, class Out>
+template <class Out>
 __device__ __forceinline__ void sell_rows_sliced(const Sell& A, const double* __restrict__ x, Out out) {
   const int lane = threadIdx.x & 31;
   const int64_t nwarps = gstride() >> 5;
@@ -313,23 +275,14 @@ __device__ __forceinline__ void sell_rows_sliced(const Sell& A, const double* __
   const uint64_t pol = evict_first_policy();
   const int64_t* __restrict__ sp = A.slice_ptr;
   const int32_t* __restrict__ col = A.col;
-  const int16_t* __restrict__ dcol = A.dcol;
   const double* __restrict__ val = A.val;
-  auto column = [&](int64_t k, int row) -> int {
-    if constexpr (kNarrow) return row + ld_stream(dcol + k, pol);
-    else if constexpr (EMG_SELL_PACKED) return ld_stream(col + packed_col_index(k), pol);
-    else return ld_stream(col + k, pol);
-  };
-  auto value = [&](int64_t k) -> double {
-    if constexpr (EMG_SELL_PACKED) return ld_stream(val + packed_val_index(k), pol);
-    else return ld_stream(val + k, pol);
-  };
+  auto column = [&](int64_t k) { return ld_stream(col + k, pol); };
+  auto value = [&](int64_t k) { return ld_stream(val + k, pol); };
   for (int64_t s = warp; s < A.nslices; s += nwarps) {
     int64_t base;
     int len;
     slice_span(sp, s, base, len);
     base += lane;
-    const int row32 = static_cast<int>(s * kSliceRows + lane);
     double sum = 0.0;
     int j = 0;
 #if EMG_SELL_PIPE == 1
@@ -345,8 +298,8 @@ __device__ __forceinline__ void sell_rows_sliced(const Sell& A, const double* __
 #pragma unroll
         for (int u = 0; u < U; ++u) {
           const bool in = jb + u < len;
-          const int64_t k = base + static_cast<int64_t>(kGroupStride) * (jb + u);
-          c[u] = in ? column(k, row32) : 0;
+          const int64_t k = base + static_cast<int64_t>(kSliceRows) * (jb + u);
+          c[u] = in ? column(k) : 0;
           v[u] = in ? value(k) : 0.0;
         }
       };
@@ -366,13 +319,13 @@ __device__ __forceinline__ void sell_rows_sliced(const Sell& A, const double* __
     }
 #endif
     for (; j + EMG_SELL_UNROLL <= len; j += EMG_SELL_UNROLL) {
-      const int64_t k = base + static_cast<int64_t>(kGroupStride) * j;
+      const int64_t k = base + static_cast<int64_t>(kSliceRows) * j;
       int c[EMG_SELL_UNROLL];
       double v[EMG_SELL_UNROLL], xv[EMG_SELL_UNROLL];
 #pragma unroll
       for (int u = 0; u < EMG_SELL_UNROLL; ++u) {
-        c[u] = column(k + kGroupStride * u, row32);
-        v[u] = value(k + kGroupStride * u);
+        c[u] = column(k + kSliceRows * u);
+        v[u] = value(k + kSliceRows * u);
       }
 #pragma unroll
       for (int u = 0; u < EMG_SELL_UNROLL; ++u) xv[u] = x[c[u]];
@@ -380,18 +333,18 @@ __device__ __forceinline__ void sell_rows_sliced(const Sell& A, const double* __
       for (int u = 0; u < EMG_SELL_UNROLL; ++u) sum += v[u] * xv[u];
     }
     for (; j < len; ++j) {
-      const int64_t k = base + static_cast<int64_t>(kGroupStride) * j;
-      sum += value(k) * x[column(k, row32)];
+      const int64_t k = base + static_cast<int64_t>(kSliceRows) * j;
+      sum += value(k) * x[column(k)];
     }
     const int64_t row = s * kSliceRows + lane;
     if (row < A.n) out(row, sum);
   }
 }
 
-template <bool kNarrow, class Out>
+template <class Out>
 __device__ __forceinline__ void sell_rows(const Sell& A, const double* __restrict__ x, Out out) {
-  if constexpr (EMG_SELL_PIPE == 2) sell_rows_stream<kNarrow>(A, x, out);
-  else sell_rows_sliced<kNarrow>(A, x, out);
+  if constexpr (EMG_SELL_PIPE == 2) sell_rows_stream(A, x, out);
+  else sell_rows_sliced(A, x, out);
 }
 
 // Same product with the slices streamed through shared memory by bulk
@@ -592,15 +545,14 @@ __device__ __forceinline__ void sell_rows_ws(const Sell& A, const double* __rest
   }
 }
 
-// Row kernels: kMode 0 = SELL with 32-bit columns, 1 = SELL with 16-bit
-// column offsets, 2 = bulk-copy pipeline (32-bit columns), 3 = warp-
+// Row kernels: kMode 0 = loads into registers, 1 = bulk-copy pipeline, 2 = warp-
 // specialized bulk-copy pipeline.
 template <int kMode, class Out>
 __device__ __forceinline__ void spmv_rows(const Sell& A, const double* __restrict__ x, Out out,
                                           int32_t* err) {
-  if constexpr (kMode == 2) sell_rows_tma(A, x, out, err);
-  else if constexpr (kMode == 3) sell_rows_ws(A, x, out, err);
-  else sell_rows<kMode == 1>(A, x, out);
+  if constexpr (kMode == 1) sell_rows_tma(A, x, out, err);
+  else if constexpr (kMode == 2) sell_rows_ws(A, x, out, err);
+  else sell_rows(A, x, out);
 }
 
 // One partial per block; true in the block that finished last (all partials
@@ -653,39 +605,16 @@ __global__ void k_sell_fill(int64_t n, int64_t nslices, const int64_t* __restric
       rl = rp[old + 1] - a;
     }
     for (int j = 0; j < len; ++j) {
-      const int64_t k = b0 + static_cast<int64_t>(kGroupStride) * j + lane;
-      const int64_t kc = EMG_SELL_PACKED ? packed_col_index(k) : k;
+      const int64_t k = b0 + static_cast<int64_t>(kSliceRows) * j + lane;
       ocol[k] = j < rl ? ccol[a + j] : 0;
       if (j < rl) {
-        col[kc] = iperm[ccol[a + j]];
+        col[k] = iperm[ccol[a + j]];
         src[k] = a + j;
       } else {
-        col[kc] = self;  // padding reads a valid entry and multiplies it by 0
+        col[k] = self;  // padding reads a valid entry and multiplies it by 0
         src[k] = -1;
       }
     }
-  }
-}
-
-// Warp per slice: dcol = col - row; *overflow = 1 if any offset leaves int16.
-__global__ void k_sell_narrow(int64_t nslices, const int64_t* __restrict__ sp,
-                              const int32_t* __restrict__ col, int16_t* __restrict__ dcol,
-                              int32_t* __restrict__ overflow) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warp = gtid() >> 5, nwarps = gstride() >> 5;
-  for (int64_t s = warp; s < nslices; s += nwarps) {
-    int64_t b0;
-    int len;
-    slice_span(sp, s, b0, len);
-    const int64_t row = s * kSliceRows + lane;
-    bool bad = false;
-    for (int j = 0; j < len; ++j) {
-      const int64_t k = b0 + static_cast<int64_t>(kGroupStride) * j + lane;
-      const int64_t d = static_cast<int64_t>(col[k]) - row;
-      bad |= d < -32768 || d > 32767;
-      dcol[k] = static_cast<int16_t>(d);
-    }
-    if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(overflow, 1);
   }
 }
 
@@ -693,7 +622,7 @@ __global__ void k_sell_values(int64_t slots, const int32_t* __restrict__ src,
                               const double* __restrict__ cval, double* __restrict__ val) {
   for (int64_t i = gtid(); i < slots; i += gstride()) {
     const int32_t s = src[i];
-    val[EMG_SELL_PACKED ? packed_val_index(i) : i] = s >= 0 ? cval[s] : 0.0;
+    val[i] = s >= 0 ? cval[s] : 0.0;
   }
 }
 
@@ -749,18 +678,18 @@ __global__ void __launch_bounds__(32) k_sell_window_perm(int64_t n, const int32_
   }
 }
 
-// Slots of every group: 32 kGroup x the longest row it holds.
-__global__ void k_sell_group_slots(int64_t n, int64_t ngroups, const int32_t* __restrict__ rp,
+// Slots of every slice: 32 x the longest row it holds.
+__global__ void k_sell_slice_slots(int64_t n, int64_t nslices, const int32_t* __restrict__ rp,
                                    const int32_t* __restrict__ perm, int32_t* __restrict__ slots) {
-  for (int64_t g = gtid(); g < ngroups; g += gstride()) {
+  for (int64_t g = gtid(); g < nslices; g += gstride()) {
     int32_t len = 0;
-    const int64_t r0 = g * kGroupStride;
-    const int64_t r1 = r0 + kGroupStride < n ? r0 + kGroupStride : n;
+    const int64_t r0 = g * kSliceRows;
+    const int64_t r1 = r0 + kSliceRows < n ? r0 + kSliceRows : n;
     for (int64_t r = r0; r < r1; ++r) {
       const int32_t o = perm[r];
       len = max(len, rp[o + 1] - rp[o]);
     }
-    slots[g] = kGroupStride * len;
+    slots[g] = kSliceRows * len;
   }
 }
 
@@ -795,11 +724,6 @@ __global__ void k_jacobi(int64_t n, const int32_t* __restrict__ rp, const int32_
   }
 }
 
-__global__ void k_gather(int64_t n, const int32_t* __restrict__ perm, const double* __restrict__ in,
-                         double* __restrict__ out) {
-  for (int64_t i = gtid(); i < n; i += gstride()) out[i] = in[perm[i]];
-}
-
 __global__ void k_scatter(int64_t n, const int32_t* __restrict__ perm, const double* __restrict__ in,
                           double* __restrict__ out) {
   for (int64_t i = gtid(); i < n; i += gstride()) out[perm[i]] = in[i];
@@ -812,7 +736,7 @@ __global__ void k_scatter(int64_t n, const int32_t* __restrict__ perm, const dou
 __global__ void __launch_bounds__(kThreads) k_product(Sell A, const int32_t* __restrict__ perm,
                                                       const double* __restrict__ x, double* __restrict__ y) {
   A.col = A.ocol;
-  sell_rows<false>(A, x, [&](int64_t row, double s) { y[perm[row]] = s; });
+  sell_rows(A, x, [&](int64_t row, double s) { y[perm[row]] = s; });
 }
 
 template <int kMode>
@@ -1410,18 +1334,17 @@ int build_sell(DevCsr& A, cudaStream_t st) {
   // its rows, a thread per slice takes the longest row, a scan gives offsets.
   const int g = grid_size();
   S.nslices = (n + kSliceRows - 1) / kSliceRows;
-  S.ngroups = (S.nslices + kGroup - 1) / kGroup;
   EMG_CK(cudaMallocAsync(&S.perm, sizeof(int32_t) * n, st));
-  EMG_CK(cudaMallocAsync(&S.slice_ptr, sizeof(int64_t) * (S.ngroups + 1), st));
+  EMG_CK(cudaMallocAsync(&S.slice_ptr, sizeof(int64_t) * (S.nslices + 1), st));
   int32_t *slice_slots = nullptr, *slice_off = nullptr;
-  EMG_CK(cudaMallocAsync(&slice_slots, sizeof(int32_t) * S.ngroups, st));
-  EMG_CK(cudaMallocAsync(&slice_off, sizeof(int32_t) * (S.ngroups + 1), st));
+  EMG_CK(cudaMallocAsync(&slice_slots, sizeof(int32_t) * S.nslices, st));
+  EMG_CK(cudaMallocAsync(&slice_off, sizeof(int32_t) * (S.nslices + 1), st));
   const int64_t windows = (n + kWindow - 1) / kWindow;
   k_sell_window_perm<<<static_cast<unsigned>(windows), 32, 0, st>>>(n, A.row_ptr, S.perm);
-  k_sell_group_slots<<<g, kThreads, 0, st>>>(n, S.ngroups, A.row_ptr, S.perm, slice_slots);
+  k_sell_slice_slots<<<g, kThreads, 0, st>>>(n, S.nslices, A.row_ptr, S.perm, slice_slots);
   EMG_CK(cudaGetLastError());
   int64_t total = 0;
-  int rc = scan_counts(slice_slots, slice_off, S.ngroups, &total, st);
+  int rc = scan_counts(slice_slots, slice_off, S.nslices, &total, st);
   if (rc) return rc;
   if (total >= (int64_t(1) << 31)) {
     cudaFreeAsync(slice_slots, st);
@@ -1429,7 +1352,7 @@ int build_sell(DevCsr& A, cudaStream_t st) {
     set_error("matrix too large for the solver format");
     return EMG_INVALID_INPUT;
   }
-  k_widen<<<g, kThreads, 0, st>>>(S.ngroups + 1, slice_off, S.slice_ptr);
+  k_widen<<<g, kThreads, 0, st>>>(S.nslices + 1, slice_off, S.slice_ptr);
   EMG_CK(cudaFreeAsync(slice_slots, st));
   EMG_CK(cudaFreeAsync(slice_off, st));
   S.slots = total;
@@ -1438,16 +1361,10 @@ int build_sell(DevCsr& A, cudaStream_t st) {
   EMG_CK(cudaMallocAsync(&iperm, sizeof(int32_t) * n, st));
   EMG_CK(cudaMallocAsync(&S.src, sizeof(int32_t) * ns, st));
   EMG_CK(cudaMallocAsync(&S.ocol, sizeof(int32_t) * ns, st));
-  if (EMG_SELL_PACKED) {  // one buffer: 32-slot chunks of values then columns
-    EMG_CK(cudaMallocAsync(&S.val, (sizeof(double) + sizeof(int32_t)) * ns, st));
-    S.col = reinterpret_cast<int32_t*>(S.val);
-  } else {
-    EMG_CK(cudaMallocAsync(&S.col, sizeof(int32_t) * ns, st));
-    EMG_CK(cudaMallocAsync(&S.val, sizeof(double) * ns, st));
-  }
+  EMG_CK(cudaMallocAsync(&S.col, sizeof(int32_t) * ns, st));
+  EMG_CK(cudaMallocAsync(&S.val, sizeof(double) * ns, st));
   k_invert_perm<<<g, kThreads, 0, st>>>(n, S.perm, iperm);
-  // every slot of every group is written: slices past the last row are padding
-  k_sell_fill<<<g, kThreads, 0, st>>>(n, S.ngroups * kGroup, S.slice_ptr, S.perm, iperm, A.row_ptr, A.col, S.col,
+  k_sell_fill<<<g, kThreads, 0, st>>>(n, S.nslices, S.slice_ptr, S.perm, iperm, A.row_ptr, A.col, S.col,
                                       S.src, S.ocol);
   EMG_CK(cudaGetLastError());
   EMG_CK(cudaFreeAsync(iperm, st));
@@ -1455,8 +1372,6 @@ int build_sell(DevCsr& A, cudaStream_t st) {
   S.max_tile_slots = 0;
   S.tma = false;
 #if EMG_SELL_TMA
-  static_assert(kGroup == 1 && !EMG_SELL_PACKED,
-                "the bulk-copy pipeline reads contiguous per-slice runs of separate arrays");
   {
     // bulk-copy pipeline: tiles of 8 slices, kStages stages in shared memory
     std::vector<int64_t> sp(S.nslices + 1);
@@ -1472,17 +1387,16 @@ int build_sell(DevCsr& A, cudaStream_t st) {
     const size_t need = tma::smem_bytes(tma::layout_for(static_cast<uint32_t>(S.max_tile_slots)));
     if (S.max_tile_slots > 0 && need <= static_cast<size_t>(optin)) {
       const int b = static_cast<int>(need);
-      EMG_CK(cudaFuncSetAttribute(k_cg_spmv_dot<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
-      EMG_CK(cudaFuncSetAttribute(k_bi_v<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
-      EMG_CK(cudaFuncSetAttribute(k_bi_t<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
-      EMG_CK(cudaFuncSetAttribute(k_spmv<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
+      EMG_CK(cudaFuncSetAttribute(k_cg_spmv_dot<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
+      EMG_CK(cudaFuncSetAttribute(k_bi_v<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
+      EMG_CK(cudaFuncSetAttribute(k_bi_t<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
+      EMG_CK(cudaFuncSetAttribute(k_spmv<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
       S.tma = true;
     }
   }
 #endif
   S.ws = false;
 #if EMG_SELL_WS
-  static_assert(kGroup == 1 && !EMG_SELL_PACKED, "the warp-specialized SpMV copies per-slice runs");
   if (!S.tma && S.nslices > 0) {
     std::vector<int64_t> sp(S.nslices + 1);
     EMG_CK(cudaMemcpyAsync(sp.data(), S.slice_ptr, sizeof(int64_t) * (S.nslices + 1), cudaMemcpyDeviceToHost, st));
@@ -1497,11 +1411,11 @@ int build_sell(DevCsr& A, cudaStream_t st) {
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (mx > 0 && need <= static_cast<size_t>(optin)) {
       const int b = static_cast<int>(need);
-      EMG_CK(cudaFuncSetAttribute(k_cg_spmv_dot<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
-      EMG_CK(cudaFuncSetAttribute(k_bi_v<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
-      EMG_CK(cudaFuncSetAttribute(k_bi_t<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
-      EMG_CK(cudaFuncSetAttribute(k_spmv<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
-      EMG_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_cg_spmv_dot<3>, kThreads, need));
+      EMG_CK(cudaFuncSetAttribute(k_cg_spmv_dot<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
+      EMG_CK(cudaFuncSetAttribute(k_bi_v<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
+      EMG_CK(cudaFuncSetAttribute(k_bi_t<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
+      EMG_CK(cudaFuncSetAttribute(k_spmv<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
+      EMG_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_cg_spmv_dot<2>, kThreads, need));
       if (per > 0) {
         S.ws = true;
         S.ws_stage_bytes = sb;
@@ -1511,28 +1425,6 @@ int build_sell(DevCsr& A, cudaStream_t st) {
     }
   }
 #endif
-  // 16-bit column offsets when every |column - row| fits (banded numberings,
-  // e.g. first-appearance edge IDs of structured meshes): 10 bytes per slot.
-  S.narrow = false;
-  if (EMG_SELL_NARROW && !EMG_SELL_PACKED && !S.tma && !S.ws && S.slots > 0) {
-    int32_t* overflow = nullptr;
-    EMG_CK(cudaMallocAsync(&S.dcol, sizeof(int16_t) * S.slots, st));
-    EMG_CK(cudaMallocAsync(&overflow, sizeof(int32_t), st));
-    EMG_CK(cudaMemsetAsync(overflow, 0, sizeof(int32_t), st));
-    k_sell_narrow<<<g, kThreads, 0, st>>>(S.nslices, S.slice_ptr, S.col, S.dcol, overflow);
-    int32_t h_over = 0;
-    EMG_CK(cudaMemcpyAsync(&h_over, overflow, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-    EMG_CK(cudaStreamSynchronize(st));
-    EMG_CK(cudaFreeAsync(overflow, st));
-    if (h_over) {
-      EMG_CK(cudaFreeAsync(S.dcol, st));
-      S.dcol = nullptr;
-    } else {
-      EMG_CK(cudaFreeAsync(S.col, st));
-      S.col = nullptr;
-      S.narrow = true;
-    }
-  }
   return EMG_SUCCESS;
 }
 
@@ -1557,9 +1449,8 @@ int ensure_sell(DevCsr& A, cudaStream_t st) {
 
 void free_sell(Sell* s) {
   if (!s) return;
-  void* col = static_cast<void*>(s->col) == static_cast<void*>(s->val) ? nullptr : static_cast<void*>(s->col);
-  for (void* p : {static_cast<void*>(s->perm), static_cast<void*>(s->slice_ptr), col,
-                  static_cast<void*>(s->dcol), static_cast<void*>(s->src), static_cast<void*>(s->ocol), static_cast<void*>(s->val)})
+  for (void* p : {static_cast<void*>(s->perm), static_cast<void*>(s->slice_ptr), static_cast<void*>(s->col),
+                  static_cast<void*>(s->src), static_cast<void*>(s->ocol), static_cast<void*>(s->val)})
     if (p) cudaFreeAsync(p, 0);
   delete s;
 }
@@ -1882,16 +1773,14 @@ int capture_loop(DevCsr& A, bool bicg, cudaGraphExec_t* out) {
 }
 
 // Launches KERNEL<mode> for the storage format of S: the bulk-copy pipeline
-// (mode 2, persistent grid + dynamic shared memory), 16-bit column offsets
-// (mode 1) or 32-bit columns (mode 0).
+// (mode 1, persistent grid + dynamic shared memory), the warp-specialized one
+// (mode 2) or loads into registers (mode 0).
 #define EMG_LAUNCH_SPMV(KERNEL, S, g, st, ...)                                        \
   do {                                                                                \
     if ((S).tma) {                                                                    \
       const SpmvShape sh_ = spmv_shape(S, g);                                         \
-      KERNEL<2><<<sh_.grid, kThreads, sh_.smem, st>>>(__VA_ARGS__);                   \
+      KERNEL<1><<<sh_.grid, kThreads, sh_.smem, st>>>(__VA_ARGS__);                   \
     } else if (EMG_WS_LAUNCH(KERNEL, S, st, __VA_ARGS__)) {                           \
-    } else if ((S).narrow) {                                                          \
-      KERNEL<1><<<sell_grid<KERNEL<1>>(S, g), kThreads, 0, st>>>(__VA_ARGS__);         \
     } else {                                                                          \
       KERNEL<0><<<sell_grid<KERNEL<0>>(S, g), kThreads, 0, st>>>(__VA_ARGS__);         \
     }                                                                                 \
@@ -1899,7 +1788,7 @@ int capture_loop(DevCsr& A, bool bicg, cudaGraphExec_t* out) {
 
 #if EMG_SELL_WS
 #define EMG_WS_LAUNCH(KERNEL, S, st, ...) \
-  ((S).ws ? (KERNEL<3><<<(S).ws_grid, kThreads, (S).ws_smem, st>>>(__VA_ARGS__), true) : false)
+  ((S).ws ? (KERNEL<2><<<(S).ws_grid, kThreads, (S).ws_smem, st>>>(__VA_ARGS__), true) : false)
 #else
 #define EMG_WS_LAUNCH(KERNEL, S, st, ...) false
 #endif
@@ -1912,15 +1801,14 @@ void tune_sell_grid(DevCsr& A, cudaStream_t st) {
   Sell& S = *A.sell;
   if (S.tma || S.ws) return;
   const int g = grid_size(), sms = num_sms();
-  const int r = S.narrow ? resident_grid<k_spmv<1>>(g) : resident_grid<k_spmv<0>>(g);
+  const int r = resident_grid<k_spmv<0>>(g);
   std::vector<int> cand{r};
   for (int d = 1; d <= 2; ++d)
     if (r - d * sms >= sms) cand.push_back(r - d * sms);
   int32_t* err = &A.ws->state->copy_err;
   const std::string key = "n" + std::to_string(A.n) + "slots" + std::to_string(S.slots);
   S.grid = tune::pick("sell.spmv_grid", key, cand, [&](int v, cudaStream_t s) {
-    if (S.narrow) k_spmv<1><<<v, kThreads, 0, s>>>(S, A.ws->p, A.ws->q, err);
-    else k_spmv<0><<<v, kThreads, 0, s>>>(S, A.ws->p, A.ws->q, err);
+    k_spmv<0><<<v, kThreads, 0, s>>>(S, A.ws->p, A.ws->q, err);
   }, st);
   cudaGetLastError();
 }
