@@ -732,11 +732,28 @@ __global__ void k_scatter(int64_t n, const int32_t* __restrict__ perm, const dou
 // y = A x in the matrix's own numbering: the slots' own columns and rows
 // written through the permutation, so a product is one launch.  (Gathering x
 // into the solvers' numbering and scattering y out of it took three launches
-// and a memset: 13.4 us for 990 rows and 65 us for the 64^3 matrix.)
+// and a memset: 13.4 us for 990 rows and 65 us for the 64^3 matrix.)  Padding
+// and masked entries multiply x[0] by 0, so a row that is no number is formed
+// again from its own entries alone (reading no x for padding in the first place
+// cost every product 2 us of 44 at 64^3).
 __global__ void __launch_bounds__(kThreads) k_product(Sell A, const int32_t* __restrict__ perm,
                                                       const double* __restrict__ x, double* __restrict__ y) {
   A.col = A.ocol;
-  sell_rows(A, x, [&](int64_t row, double s) { y[perm[row]] = s; });
+  sell_rows(A, x, [&](int64_t row, double s) {
+    if (!isfinite(s)) {
+      int64_t base;
+      int len;
+      slice_span(A.slice_ptr, row / kSliceRows, base, len);
+      base += row % kSliceRows;
+      s = 0.0;
+#pragma unroll 1  // unrolled it takes 74 registers, a block less an SM
+      for (int j = 0; j < len; ++j) {
+        const int64_t k = base + static_cast<int64_t>(kSliceRows) * j;
+        if (A.src[k] >= 0) s += A.val[k] * x[A.ocol[k]];
+      }
+    }
+    y[perm[row]] = s;
+  });
 }
 
 template <int kMode>
