@@ -1925,6 +1925,7 @@ int run_solver(DevCsr& A, const double* b, double* x, const emg_krylov_config& c
     EMG_CK(cudaEventRecord(w.ev1, st));
     EMG_CK(cudaMemcpyAsync(w.state_h, w.state, sizeof(SolverState), cudaMemcpyDeviceToHost, st));
     EMG_CK(cudaStreamSynchronize(st));
+    if (w.state_h->copy_err) w.state_h->status = EMG_ERR_TIMEOUT;  // one block's wait ran out: its x is not the others'
     return finish_solver(w, w.state_h->done != 0, res);
   }
   // Preferred: the whole solve as one graph with a device while-loop; else

@@ -54,7 +54,8 @@ struct ResidentArgs {
 // published to k - 1; and the reset is seen before anything is polled there,
 // since one of the reductions k .. k + 2 carries the fence in every sequence
 // the kernels run (CG alternates, BiCGSTAB has two without in a row at most).
-// False when a wait ran out.
+// False when a wait ran out: the block raises st->copy_err at its end and the solve
+// counts as timed out, whatever the other blocks had seen by then.
 template <int T>
 struct GridSums {
   unsigned long long* slots;
@@ -282,6 +283,7 @@ __global__ void __launch_bounds__(T, 1) k_cg_resident(ResidentArgs P) {
 #pragma unroll
   for (int q = 0; q < NR; ++q)
     if (R.live[q]) P.x[P.A.perm[R.row[q]]] = x[q];
+  if (threadIdx.x == 0 && sh_bad) atomicOr(&P.st->copy_err, 1);
   if (writer) {
     P.st->status = status;
     P.st->iter = it;
@@ -391,6 +393,7 @@ __global__ void __launch_bounds__(T, 1) k_bi_resident(ResidentArgs P) {
 #pragma unroll
   for (int q = 0; q < NR; ++q)
     if (R.live[q]) P.x[P.A.perm[R.row[q]]] = x[q];
+  if (threadIdx.x == 0 && sh_bad) atomicOr(&P.st->copy_err, 1);
   if (writer) {
     P.st->status = status;
     P.st->iter = it;
