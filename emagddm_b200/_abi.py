@@ -95,6 +95,7 @@ SIGNATURES = {
                           C.POINTER(Result)], C.c_int),
     "emg_cg_kernel_times": ([H, C.c_int32, VP, VP], C.c_int),
     "emg_test_set_barrier_spins": ([C.c_int32], C.c_int),
+    "emg_test_set_resident": ([C.c_int32], C.c_int),
     "emg_tune_enable": ([C.c_int32], C.c_int),
     "emg_aedt_read": ([C.c_char_p, C.POINTER(H)], C.c_int),
     "emg_aedt_info": ([H, C.POINTER(C.c_int32), C.POINTER(C.c_int32), C.POINTER(C.c_int32)], C.c_int),

@@ -827,6 +827,11 @@ int emg_test_set_barrier_spins(int32_t spins) {
   return guarded([&]() -> int { return emg::set_barrier_spins(spins); });
 }
 
+int emg_test_set_resident(int32_t on) {
+  emg::set_resident(on != 0);
+  return EMG_SUCCESS;
+}
+
 int emg_batch_cg_solve_device(emg_csr A, int32_t n_blocks, const int64_t* block_row_ptr,
                               const double* b_d, double* x_d, const emg_krylov_config* cfg,
                               void* stream, emg_result* results) {

@@ -24,6 +24,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -1637,6 +1638,7 @@ void launch_update_dir(KrylovWorkspace& w, int64_t n, cudaStream_t st) {
 // 46.2 but 46^3 76.4 against 61.7 (the vectors spill and the matrix is read
 // through L2 at a quarter of the graph kernels' occupancy).
 constexpr int64_t kResMinSlices = 8;
+std::atomic<bool> g_resident{true};  // a test turns it off to run small matrices through the loop graph
 using ResidentKernel = void (*)(ResidentArgs);
 struct ResidentShape {
   int threads, rows;
@@ -1921,7 +1923,7 @@ int run_solver(DevCsr& A, const double* b, double* x, const emg_krylov_config& c
   EMG_CK(cudaMemcpyAsync(w.state, w.state_h, sizeof(SolverState), cudaMemcpyHostToDevice, st));
   const int g = w.grid;
   bool done = false;
-  if (w.res_grid > 0 && launch_resident(A, b, x, cfg.preconditioner, bicg, st)) {
+  if (w.res_grid > 0 && g_resident && launch_resident(A, b, x, cfg.preconditioner, bicg, st)) {
     EMG_CK(cudaEventRecord(w.ev1, st));
     EMG_CK(cudaMemcpyAsync(w.state_h, w.state, sizeof(SolverState), cudaMemcpyDeviceToHost, st));
     EMG_CK(cudaStreamSynchronize(st));
@@ -2021,6 +2023,8 @@ int set_barrier_spins(int32_t spins) {
   EMG_CK(cudaMemcpyToSymbol(g_barrier_spins, &v, sizeof(v)));
   return EMG_SUCCESS;
 }
+
+void set_resident(bool on) { g_resident = on; }
 
 int cg_kernel_times(DevCsr& A, int32_t iterations, cudaStream_t user, double* ms) {
   if (iterations <= 0 || !ms) { set_error("bad arguments"); return EMG_INVALID_INPUT; }

@@ -485,11 +485,16 @@ int emg_tune_enable(int32_t on);
 int32_t emg_tune_report(char* buf, int32_t cap);
 
 /* Test hook (no counterpart in the reference): polls a block of the fused
- * CG update makes at its grid barrier before giving up (default 2^21, about
+ * CG update or of a resident solve makes at its grid barrier before giving up (default 2^21, about
  * 0.2 s or more; a negative value restores it) on the current device.  A
  * block that gives up ends the solve with EMG_ERR_TIMEOUT instead of
  * waiting on; tests lower the limit to make that wait run out. */
 int emg_test_set_barrier_spins(int32_t spins);
+
+/* Test hook (no counterpart in the reference): 0 keeps CG and BiCGSTAB solves
+ * off the kernel that runs a small matrix's whole solve, so tests can put small
+ * matrices through the loop of larger ones; 1 (the default) restores it. */
+int emg_test_set_resident(int32_t on);
 
 /* Test hook (no counterpart in the reference): one tile of the
  * mixed-precision factor's tensor-core contraction, C -= A B^T with A
