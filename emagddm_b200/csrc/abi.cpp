@@ -824,7 +824,10 @@ int32_t emg_tune_report(char* buf, int32_t cap) {
 }
 
 int emg_test_set_barrier_spins(int32_t spins) {
-  return guarded([&]() -> int { return emg::set_barrier_spins(spins); });
+  return guarded([&]() -> int {
+    const int rc = emg::set_barrier_spins(spins);
+    return rc ? rc : emg::set_front_polls(spins);
+  });
 }
 
 int emg_test_set_resident(int32_t on) {
@@ -922,7 +925,7 @@ int fetidp_solve_impl(emg::FetiDP* fp, const emg_krylov_config* cfg, const doubl
   }
   emg_result r{};
   int rc = F.solve(*cfg, bd, on_device ? x : nullptr, &r);
-  if (rc == EMG_SUCCESS || rc == EMG_MAX_ITER_REACHED || rc == EMG_NUMERICAL_ERROR) {
+  if (rc == EMG_SUCCESS || rc == EMG_MAX_ITER_REACHED || rc == EMG_NUMERICAL_ERROR || rc == EMG_ERR_TIMEOUT) {
     if (x && !on_device) {
       cudaError_t e = cudaMemcpy(x, F.xacc_d, sizeof(double) * n, cudaMemcpyDeviceToHost);
       if (e != cudaSuccess) { set_error(cudaGetErrorString(e)); return EMG_ERR_CUDA; }

@@ -1043,7 +1043,10 @@ __global__ void __launch_bounds__(kPivMax) k_front_bwd_piv(FrontsDev F, int32_t 
 // side took 14.1 ms on the 24^3 direct factor (two passes over the fronts);
 // one pass takes 7.0 ms there and 1.1 ms here.
 constexpr int kRB = kNB;  // rows of a block
-constexpr int kWaitPolls = 1 << 22;
+constexpr int32_t kWaitPolls = 1 << 22;
+// Polls a waiting block of the front solves and of the root products makes before
+// it gives up; kWaitPolls unless a test lowers it (emg_test_set_barrier_spins).
+__device__ int32_t g_wait_polls = kWaitPolls;
 
 __device__ __forceinline__ int32_t ld_acquire(const int32_t* p) {
   int32_t v;
@@ -1055,8 +1058,8 @@ __device__ __forceinline__ void st_release(int32_t* p, int32_t v) {
 }
 
 // Waits until *p >= want; the last value seen, or -1 when the wait ran out.
-__device__ __forceinline__ int32_t wait_progress(const int32_t* p, int32_t want) {
-  for (int i = 0; i < kWaitPolls; ++i) {
+__device__ __forceinline__ int32_t wait_progress(const int32_t* p, int32_t want, int32_t polls) {
+  for (int32_t i = 0; i < polls; ++i) {
     const int32_t v = ld_acquire(p);
     if (v >= want) return v;
   }
@@ -1070,6 +1073,7 @@ __global__ void __launch_bounds__(256) k_front_fwd_rows(FrontsDev F, int32_t f0,
   __shared__ double xs[kRB], vs[kRB], ys[2][kRB], part[4][kRB];
   __shared__ double X[kRB][kRB + 1];  // X[r][c] = (L_II^-1)(r, c)
   const int t = threadIdx.x, r = t & (kRB - 1), g = t >> 6;
+  const int32_t polls = g_wait_polls;
   if (t == 0) tk = atomicAdd(ticket, 1);
   __syncthreads();
   const int32_t b = tk / nf, k = f0 + (tk - b * nf);
@@ -1122,9 +1126,9 @@ __global__ void __launch_bounds__(256) k_front_fwd_rows(FrontsDev F, int32_t f0,
     for (int c = 0; c < 16; ++c) lc[c] = ln[c];
     if (J + 1 < nt) fetch(J + 1);
     if (t < kRB) {
-      if (seen <= J) seen = wait_progress(prog + k, J + 1);
+      if (seen <= J) seen = wait_progress(prog + k, J + 1, polls);
       if (seen < 0) {
-        if (t == 0) atomicOr(err, kErrWait);
+        atomicOr(err, kErrWait);
         seen = INT32_MAX;
         acc = nan("");
       }
@@ -1163,6 +1167,7 @@ __global__ void __launch_bounds__(256) k_front_bwd_rows(FrontsDev F, int32_t f0,
   __shared__ int32_t tk;
   __shared__ double dots[kRB], vs[kRB], part[4][kRB];
   const int t = threadIdx.x, lane = t & 31, w = t >> 5, r = t & (kRB - 1), g = t >> 6;
+  const int32_t polls = g_wait_polls;
   if (t == 0) tk = atomicAdd(ticket, 1);
   __syncthreads();
   const int32_t q = tk / nf, k = f0 + (tk - q * nf);
@@ -1219,9 +1224,9 @@ __global__ void __launch_bounds__(256) k_front_bwd_rows(FrontsDev F, int32_t f0,
 #pragma unroll
     for (int c = 0; c < 8; ++c) { l0[c] = n0[c]; l1[c] = n1[c]; }
     if (I - 1 > J) fetch(I - 1);
-    if (seen < nbp - I) seen = wait_progress(prog + k, nbp - I);
+    if (seen < nbp - I) seen = wait_progress(prog + k, nbp - I, polls);
     if (seen < 0) {
-      if (lane == 0) atomicOr(err, kErrWait);
+      atomicOr(err, kErrWait);
       seen = INT32_MAX;
       acc[0] = nan("");
     }
@@ -1600,7 +1605,7 @@ struct TriSmem {
 
 template <bool kInverse, int kK, int kR, class T>
 __device__ __forceinline__ bool tri_rows(const T* __restrict__ M, int64_t off, int32_t n, int32_t ra, int32_t rb,
-                                         const TriSmem& sm, uint32_t& phase, uint64_t pol,
+                                         const TriSmem& sm, uint32_t& phase, uint64_t pol, uint32_t polls,
                                          double2* __restrict__ out) {
   static_assert(kR <= 8 && kTriT == 512, "a lane adds kR / 2 of the 16 warps' values");
   constexpr int V = 16 / sizeof(T);
@@ -1623,7 +1628,7 @@ __device__ __forceinline__ bool tri_rows(const T* __restrict__ M, int64_t off, i
     for (int i = 0; i < min(depth, steps); ++i) fetch(i, i);
   double acc[kK] = {};
   for (int i = 0, stage = 0, buf = 0; i < steps; ++i, buf ^= 1) {
-    const bool ok = tma::mbar_wait(sm.full + stage, (phase >> stage) & 1u);
+    const bool ok = tma::mbar_wait(sm.full + stage, (phase >> stage) & 1u, polls);
     const int32_t r = ra + i * kR;
     double v[kR][kK], s[kR];
 #pragma unroll
@@ -1713,6 +1718,7 @@ __global__ void __launch_bounds__(kTriT, 1) k_tri_apply(const TriSeg* __restrict
   if (threadIdx.x < kTriStages) tma::mbar_init(sm.full + threadIdx.x, 1);
   tma::fence_mbar_init();
   const uint64_t pol = evict_first_policy();
+  const uint32_t polls = static_cast<uint32_t>(g_wait_polls);
   uint32_t phase = 0;
   bool ok = true;
   for (int32_t g = cta_seg[blockIdx.x]; g < cta_seg[blockIdx.x + 1]; ++g) {
@@ -1728,14 +1734,14 @@ __global__ void __launch_bounds__(kTriT, 1) k_tri_apply(const TriSeg* __restrict
       tma::fence_proxy_async();
       __syncthreads();
       switch (kk) {
-        case 1: ok = tri_rows<kInverse, 1, 8>(M, o, n, S.ra, S.rb, sm, phase, pol, out); break;
-        case 2: ok = tri_rows<kInverse, 2, 8>(M, o, n, S.ra, S.rb, sm, phase, pol, out); break;
-        case 3: ok = tri_rows<kInverse, 3, 8>(M, o, n, S.ra, S.rb, sm, phase, pol, out); break;
-        case 4: ok = tri_rows<kInverse, 4, 4>(M, o, n, S.ra, S.rb, sm, phase, pol, out); break;
-        case 5: ok = tri_rows<kInverse, 5, 4>(M, o, n, S.ra, S.rb, sm, phase, pol, out); break;
-        case 6: ok = tri_rows<kInverse, 6, 4>(M, o, n, S.ra, S.rb, sm, phase, pol, out); break;
-        case 7: ok = tri_rows<kInverse, 7, 2>(M, o, n, S.ra, S.rb, sm, phase, pol, out); break;
-        default: ok = tri_rows<kInverse, kTriMaxK, 2>(M, o, n, S.ra, S.rb, sm, phase, pol, out); break;
+        case 1: ok = tri_rows<kInverse, 1, 8>(M, o, n, S.ra, S.rb, sm, phase, pol, polls, out); break;
+        case 2: ok = tri_rows<kInverse, 2, 8>(M, o, n, S.ra, S.rb, sm, phase, pol, polls, out); break;
+        case 3: ok = tri_rows<kInverse, 3, 8>(M, o, n, S.ra, S.rb, sm, phase, pol, polls, out); break;
+        case 4: ok = tri_rows<kInverse, 4, 4>(M, o, n, S.ra, S.rb, sm, phase, pol, polls, out); break;
+        case 5: ok = tri_rows<kInverse, 5, 4>(M, o, n, S.ra, S.rb, sm, phase, pol, polls, out); break;
+        case 6: ok = tri_rows<kInverse, 6, 4>(M, o, n, S.ra, S.rb, sm, phase, pol, polls, out); break;
+        case 7: ok = tri_rows<kInverse, 7, 2>(M, o, n, S.ra, S.rb, sm, phase, pol, polls, out); break;
+        default: ok = tri_rows<kInverse, kTriMaxK, 2>(M, o, n, S.ra, S.rb, sm, phase, pol, polls, out); break;
       }
     }
     if (!ok) {
@@ -2696,6 +2702,12 @@ int FetiDP::setup_device() {
   return EMG_SUCCESS;
 }
 
+int set_front_polls(int32_t polls) {
+  const int32_t v = polls < 0 ? kWaitPolls : polls;
+  EMG_CK(cudaMemcpyToSymbol(g_wait_polls, &v, sizeof(v)));
+  return EMG_SUCCESS;
+}
+
 int FetiDP::check_err(const char* where) {
   int32_t e = 0;
   EMG_CK(cudaMemcpyAsync(&e, err_d, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
@@ -2707,7 +2719,7 @@ int FetiDP::check_err(const char* where) {
     return EMG_NUMERICAL_ERROR;
   }
   if (e & kErrWait) {
-    set_error(std::string(where) + ": a front solve gave up waiting for a block of its front");
+    set_error(std::string(where) + ": a front solve or a root product gave up waiting");
     return EMG_ERR_TIMEOUT;
   }
   if (e & kErrTc) {
@@ -3529,6 +3541,14 @@ int FetiDP::apply_op(int32_t op, const double* in, double* out) {
   const int32_t saved = precond;
   precond = 2;
   int rc = EMG_SUCCESS;
+  // under capture a wait that runs out shows as NaN in out alone
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) {
+    cudaGetLastError();
+    cs = cudaStreamCaptureStatusActive;
+  }
+  const bool eager = cs == cudaStreamCaptureStatusNone;
+  if (eager) EMG_CK(cudaMemsetAsync(err_d, 0, sizeof(int32_t), st));
   if (op == 0) apply_F(in, out, part_d);
   else if (op == 1) apply_M(in, out, part_d);
   else if (op == 2) rc = learned_apply(*this, in, nullptr, out);
@@ -3541,6 +3561,7 @@ int FetiDP::apply_op(int32_t op, const double* in, double* out) {
   }
   precond = saved;
   if (!rc) EMG_CK(cudaGetLastError());
+  if (!rc && eager) rc = check_err("FETI-DP multiplier operator");
   return rc;
 }
 
@@ -3550,12 +3571,12 @@ int FetiDP::lambda_rhs(const double* b, double* out) {
   if (b) EMG_CK(cudaMemcpyAsync(bg_d, b, sizeof(double) * N, cudaMemcpyDeviceToDevice, st));
   else k_gather_sum<int32_t><<<blocks_for(N, 256), 256, 0, st>>>(N, d_gptr, d_glist, un.rhs, bg_d);
   k_distribute<<<blocks_for(N, 256), 256, 0, st>>>(N, d_gptr, d_glist, bg_d, fu_d);
+  EMG_CK(cudaMemsetAsync(err_d, 0, sizeof(int32_t), st));
   int rc = prepare_rhs(fu_d);
   if (rc) return rc;
   if (plan.n_lambda > 0)
     EMG_CK(cudaMemcpyAsync(out, rhs_d, sizeof(double) * plan.n_lambda, cudaMemcpyDeviceToDevice, st));
-  EMG_CK(cudaStreamSynchronize(st));
-  return EMG_SUCCESS;
+  return check_err("FETI-DP right-hand side");  // synchronizes
 }
 
 // Recovery for the union right-hand side fu into xg_d:
@@ -3718,6 +3739,7 @@ int FetiDP::solve(const emg_krylov_config& cfg, const double* b_d, double* x_d, 
   const int64_t N = P.n_dofs;
   EventPair ev;
   EMG_CK(cudaEventRecord(ev.a, st));
+  EMG_CK(cudaMemsetAsync(err_d, 0, sizeof(int32_t), st));
   // global right-hand side: the assembled F, or the caller's vector
   if (b_d) EMG_CK(cudaMemcpyAsync(bg_d, b_d, sizeof(double) * N, cudaMemcpyDeviceToDevice, st));
   else k_gather_sum<int32_t><<<blocks_for(N, 256), 256, 0, st>>>(N, d_gptr, d_glist, un.rhs, bg_d);
@@ -3771,7 +3793,6 @@ int FetiDP::solve(const emg_krylov_config& cfg, const double* b_d, double* x_d, 
     double rr = 0.0;
     rc = global_residual(bg_d, xacc_d, &rr);
     if (rc) return rc;
-    if (!std::isfinite(rr) && (rc = check_err("FETI-DP solve"))) return rc;  // a front solve's wait ran out
     {  // global_residual synchronized the stream: all four events are complete
       float a = 0.f, b = 0.f, c = 0.f;
       cudaEventElapsedTime(&a, ph0.a, ph0.b);
@@ -3781,6 +3802,10 @@ int FetiDP::solve(const emg_krylov_config& cfg, const double* b_d, double* x_d, 
       lambda_ms += b;
     }
     const double rel_new = std::sqrt(rr / bb);
+    if (!std::isfinite(rr) && (rc = check_err("FETI-DP solve"))) {  // no further passes of waits that run out
+      status = rc;
+      break;
+    }
     if (status == EMG_NUMERICAL_ERROR) break;
     if (!(rel_new < 0.5 * rel)) {
       // the pass did not pay: undo it and retry with a much tighter tolerance
@@ -3798,6 +3823,9 @@ int FetiDP::solve(const emg_krylov_config& cfg, const double* b_d, double* x_d, 
     if (total >= cfg.max_iterations) break;
   }
   if (bb > 0.0 && status == EMG_SUCCESS && !(rel < cfg.tolerance)) status = EMG_MAX_ITER_REACHED;
+  // a wait that ran out poisons what it waited for, so no such solve ends in success
+  if (status != EMG_SUCCESS)
+    if (const int rc = check_err("FETI-DP solve")) status = rc;
   EMG_CK(cudaEventRecord(ev.b, st));
   if (x_d) EMG_CK(cudaMemcpyAsync(x_d, xacc_d, sizeof(double) * N, cudaMemcpyDeviceToDevice, st));
   EMG_CK(cudaStreamSynchronize(st));

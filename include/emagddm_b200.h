@@ -484,11 +484,13 @@ int emg_tune_enable(int32_t on);
  * length needed including the NUL. */
 int32_t emg_tune_report(char* buf, int32_t cap);
 
-/* Test hook (no counterpart in the reference): polls a block of the fused
- * CG update or of a resident solve makes at its grid barrier before giving up (default 2^21, about
- * 0.2 s or more; a negative value restores it) on the current device.  A
- * block that gives up ends the solve with EMG_ERR_TIMEOUT instead of
- * waiting on; tests lower the limit to make that wait run out. */
+/* Test hook (no counterpart in the reference): polls that a waiting block
+ * makes before it gives up, at the grid barrier of the fused CG update and of
+ * the resident solves (default 2^21, about 0.2 s or more) and in the front
+ * solves and root products of FETI-DP and the direct solver (2^22); a negative
+ * value restores the defaults.  On the current device.  A block that gives up
+ * ends the solve with EMG_ERR_TIMEOUT instead of waiting on; tests lower the
+ * limit to make these waits run out. */
 int emg_test_set_barrier_spins(int32_t spins);
 
 /* Test hook (no counterpart in the reference): 0 keeps CG and BiCGSTAB solves
