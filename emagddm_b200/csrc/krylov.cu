@@ -757,12 +757,6 @@ __global__ void __launch_bounds__(kThreads) k_product(Sell A, const int32_t* __r
   });
 }
 
-template <int kMode>
-__global__ void __launch_bounds__(kThreads) k_spmv(Sell A, const double* __restrict__ x,
-                                                   double* __restrict__ y, int32_t* err) {
-  spmv_rows<kMode>(A, x, [&](int64_t row, double s) { y[row] = s; }, err);
-}
-
 // ----------------------------------------------------------------- CG ----
 __global__ void __launch_bounds__(kThreads) k_cg_init(int64_t n, const double* __restrict__ b,
                                                       const int32_t* __restrict__ perm,
@@ -1408,7 +1402,6 @@ int build_sell(DevCsr& A, cudaStream_t st) {
       EMG_CK(cudaFuncSetAttribute(k_cg_spmv_dot<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
       EMG_CK(cudaFuncSetAttribute(k_bi_v<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
       EMG_CK(cudaFuncSetAttribute(k_bi_t<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
-      EMG_CK(cudaFuncSetAttribute(k_spmv<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
       S.tma = true;
     }
   }
@@ -1432,7 +1425,6 @@ int build_sell(DevCsr& A, cudaStream_t st) {
       EMG_CK(cudaFuncSetAttribute(k_cg_spmv_dot<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
       EMG_CK(cudaFuncSetAttribute(k_bi_v<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
       EMG_CK(cudaFuncSetAttribute(k_bi_t<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
-      EMG_CK(cudaFuncSetAttribute(k_spmv<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
       EMG_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_cg_spmv_dot<2>, kThreads, need));
       if (per > 0) {
         S.ws = true;
@@ -1812,22 +1804,22 @@ int capture_loop(DevCsr& A, bool bicg, cudaGraphExec_t* out) {
 #define EMG_WS_LAUNCH(KERNEL, S, st, ...) false
 #endif
 
-// Blocks per SM of the register-pipeline SpMV (the SELL kernel without the
-// solver's dot product, whose loads and occupancy are the same), chosen by
-// the autotuner for this matrix shape: one resident wave (the default) or
-// one or two blocks per SM fewer, timed on the matrix itself.
+// Blocks per SM of the register-pipeline SpMV, chosen by the autotuner for this
+// matrix shape: one resident wave (the default) or one or two blocks per SM
+// fewer, timed with the product (k_product, whose loads and occupancy the loop
+// graph's kernels share) on the matrix itself.
 void tune_sell_grid(DevCsr& A, cudaStream_t st) {
   Sell& S = *A.sell;
   if (S.tma || S.ws) return;
   const int g = grid_size(), sms = num_sms();
-  const int r = resident_grid<k_spmv<0>>(g);
+  const int r = resident_grid<k_product>(g);
   std::vector<int> cand{r};
   for (int d = 1; d <= 2; ++d)
     if (r - d * sms >= sms) cand.push_back(r - d * sms);
-  int32_t* err = &A.ws->state->copy_err;
   const std::string key = "n" + std::to_string(A.n) + "slots" + std::to_string(S.slots);
+  cudaMemsetAsync(A.ws->p, 0, sizeof(double) * A.n, st);  // no rows that are no number
   S.grid = tune::pick("sell.spmv_grid", key, cand, [&](int v, cudaStream_t s) {
-    k_spmv<0><<<v, kThreads, 0, s>>>(S, A.ws->p, A.ws->q, err);
+    k_product<<<v, kThreads, 0, s>>>(S, S.perm, A.ws->p, A.ws->q);
   }, st);
   cudaGetLastError();
 }
