@@ -2858,26 +2858,31 @@ int FetiDP::trtri(int32_t n_mat, int32_t max_n, const int32_t* dim, const int64_
   return EMG_SUCCESS;
 }
 
+// Largest pivot and update counts and fronts of every level (once).
+void FetiDP::front_levels() {
+  const int32_t nlev = static_cast<int32_t>(plan.level_ptr.size()) - 1;
+  if (static_cast<int32_t>(lvl_max_np.size()) == nlev) return;
+  lvl_max_np.assign(nlev, 0);
+  lvl_max_nu.assign(nlev, 0);
+  lvl_max_f.assign(nlev, 0);
+  lvl_max_blk.assign(nlev, 0);
+  for (int32_t h = 0; h < nlev; ++h)
+    for (int32_t k = plan.level_ptr[h]; k < plan.level_ptr[h + 1]; ++k) {
+      const FetiFront& x = plan.fronts[k];
+      if (x.is_root) continue;
+      lvl_max_np[h] = std::max(lvl_max_np[h], x.npiv);
+      lvl_max_nu[h] = std::max(lvl_max_nu[h], x.f - x.npiv);
+      lvl_max_f[h] = std::max(lvl_max_f[h], x.f);
+      lvl_max_blk[h] = std::max(lvl_max_blk[h], (x.npiv + kRB - 1) / kRB + (x.f - x.npiv + kRB - 1) / kRB);
+    }
+}
+
 // Multifrontal forward / backward solve of K_rr x = b for ncol right-hand
 // sides: blocked front kernels level by level, the root (dual) fronts with
 // their explicit inverse factors.
 int FetiDP::solve_fronts(const RhsDev& R, int32_t ncol) {
   const int32_t nlev = static_cast<int32_t>(plan.level_ptr.size()) - 1;
-  if (static_cast<int32_t>(lvl_max_np.size()) != nlev) {  // largest pivot / update counts per level
-    lvl_max_np.assign(nlev, 0);
-    lvl_max_nu.assign(nlev, 0);
-    lvl_max_f.assign(nlev, 0);
-    lvl_max_blk.assign(nlev, 0);
-    for (int32_t h = 0; h < nlev; ++h)
-      for (int32_t k = plan.level_ptr[h]; k < plan.level_ptr[h + 1]; ++k) {
-        const FetiFront& x = plan.fronts[k];
-        if (x.is_root) continue;
-        lvl_max_np[h] = std::max(lvl_max_np[h], x.npiv);
-        lvl_max_nu[h] = std::max(lvl_max_nu[h], x.f - x.npiv);
-        lvl_max_f[h] = std::max(lvl_max_f[h], x.f);
-        lvl_max_blk[h] = std::max(lvl_max_blk[h], (x.npiv + kRB - 1) / kRB + (x.f - x.npiv + kRB - 1) / kRB);
-      }
-  }
+  front_levels();
   const unsigned nc = static_cast<unsigned>(ncol);
   const unsigned ngroups = static_cast<unsigned>((ncol + kColB - 1) / kColB);
   const unsigned ngroups_mid = static_cast<unsigned>((ncol + kMidCols - 1) / kMidCols);
@@ -3170,7 +3175,8 @@ int FetiDP::factor(const double* nu, const double* sigma, int32_t n_mat, const e
   EMG_CK(cudaGetLastError());
   EMG_CK(cudaEventRecord(ev.b, st));
   EMG_CK(cudaEventSynchronize(ev.b));
-  stats.factor_ms = ev.ms();
+  stats.factor_ms = ev.ms() - tune_ms;
+  tune_ms = 0.0;
   factored = true;
   if (!tuned) {  // once per solver, after its first factorization (not in factor_ms)
     tuned = true;
@@ -3252,8 +3258,9 @@ int FetiDP::factor_device() {
   const int64_t nc = P.n_coarse;
   if (nc > 0) {  // without a coarse problem (the direct solver) nothing reads Phi
     // Phi = K_rr^-1 K_rP (columns 0..nP-1) and z = K_rr^-1 f_r (column nP)
-    EMG_CK(cudaMemsetAsync(phi_d, 0, sizeof(double) * std::max<int64_t>(phi_size, 1), st));
     RhsDev R{phi_d, d_roff_s, d_ncol_s, d_voff_s, vs_d};
+    if (!tuned && !capturing) tune_front_solves(R);
+    EMG_CK(cudaMemsetAsync(phi_d, 0, sizeof(double) * std::max<int64_t>(phi_size, 1), st));
     k_setup_rhs<<<dim3(64, static_cast<unsigned>(S)), 256, 0, st>>>(d_loc_off, d_nI, d_nD, d_nP, rp, cl, vl, un.rhs,
                                                                      R);
     rc = solve_fronts(R, max_ncol);
@@ -3290,34 +3297,49 @@ int FetiDP::factor_device() {
   return EMG_SUCCESS;
 }
 
-// Launch choices of the solve kernels, made by the autotuner on this plan's
-// shape (tune.h): the fused kernels on the medium-front levels or not, the
-// CTA widths of the pivot-block and update-row kernels of the front
-// solves (a single-column solve into scratch vectors) and of the dense column
-// dots of the multiplier iteration (an S_DD pass).  The values of the
-// vectors do not matter for the timing; the kernels read and write only the
-// solver's own scratch.
-void FetiDP::tune_solve_kernels() {
-  const std::string key = "u" + std::to_string(plan.n_union) + "f" + std::to_string(plan.fronts.size()) + "s" +
-                          std::to_string(plan.n_parts);
-  // the two-kernel front solves run on multi-column solves only (the coarse
-  // basis): timed on the level of the largest fronts, one column
+std::string FetiDP::tune_key() const {
+  return "u" + std::to_string(plan.n_union) + "f" + std::to_string(plan.fronts.size()) + "s" +
+         std::to_string(plan.n_parts);
+}
+
+// Launch choices made by the autotuner on this plan's shape (tune.h).  The
+// values of the vectors do not matter for the timing; the kernels read and
+// write only the solver's own scratch.
+//   The CTA widths of the pivot-block and update-row kernels, which only the
+// coarse basis takes (several columns, levels of large fronts): timed on the
+// level of the largest fronts with one group of columns, before the basis is
+// formed in the same arrays.
+void FetiDP::tune_front_solves(const RhsDev& R) {
+  front_levels();
+  EventPair ev;
+  cudaEventRecord(ev.a, st);
+  const std::string key = tune_key();
   int32_t top = -1;
   for (size_t h = 0; h < lvl_max_np.size(); ++h)
     if (lvl_max_np[h] > 0 && lvl_max_nu[h] > 0 && (top < 0 || lvl_max_f[h] > lvl_max_f[top])) top = static_cast<int32_t>(h);
-  if (top >= 0 && n_roots > 0) {
-    RhsDev R1{xu_d, d_roff1, d_ncol1, d_voff1, v1_d};
+  if (top >= 0) {
+    const unsigned nc = static_cast<unsigned>(std::min<int32_t>(kColB, max_ncol));
     const int32_t f0 = plan.level_ptr[top];
     const unsigned nf = static_cast<unsigned>(plan.level_ptr[top + 1] - f0);
     piv_threads = tune::pick("feti.front_pivot_threads", key, {512, 256, 1024}, [&](int v, cudaStream_t) {
-      k_front_fwd_piv<<<dim3(1, nf), v, 0, st>>>(fd, f0, R1, d_nI, d_nD, fac_d);
+      k_front_fwd_piv<<<dim3(nc, nf), v, 0, st>>>(fd, f0, R, d_nI, d_nD, fac_d);
     }, st);
     const int32_t saved_upd = upd_rows;
     upd_rows = tune::pick("feti.front_update_rows", key, {saved_upd, 128, 512}, [&](int v, cudaStream_t) {
       k_front_fwd_upd<<<dim3(static_cast<unsigned>((lvl_max_nu[top] + v - 1) / v), nf, 1), v, 0, st>>>(
-          fd, f0, R1, d_nI, d_nD, fac_d);
+          fd, f0, R, d_nI, d_nD, fac_d);
     }, st);
   }
+  cudaEventRecord(ev.b, st);
+  cudaEventSynchronize(ev.b);
+  cudaGetLastError();
+  tune_ms = ev.ms();
+}
+
+// The width of the dense column dots of the multiplier iteration (an S_DD
+// pass), after the first factorization.
+void FetiDP::tune_solve_kernels() {
+  const std::string key = tune_key();
   if (n_roots > 0)
     gemv_warps = tune::pick("feti.dense_column_warps", key, {8, 4, 16}, [&](int v, cudaStream_t) {
       const dim3 gr(static_cast<unsigned>((max_nD + v - 1) / v), static_cast<unsigned>(n_roots));

@@ -85,6 +85,7 @@ struct FetiDP {
   // CTA widths of the solve kernels (autotuned after the first factorization)
   int32_t piv_threads = 512, upd_rows = 256, gemv_warps = 8;
   bool tuned = false;
+  double tune_ms = 0.0;  // device time of the tuning inside the first factorization
   int32_t precond = 2;  // 0 none, 1 Dirichlet stiffness-scaled, 2 deluxe-scaled, 3 deluxe with FP32 blocks,
                         // 4 deluxe + learned correction (flexible CG)
   FetiStats stats;
@@ -199,6 +200,9 @@ struct FetiDP {
   void apply_M(const double* r, double* z, double* part);
   int dot(const double* a, const double* b, int64_t n, int which);
   int setup_deluxe();
+  void front_levels();
+  std::string tune_key() const;
+  void tune_front_solves(const RhsDev& R);
   void tune_solve_kernels();
   int trtri(int32_t n_mat, int32_t max_n, const int32_t* dim, const int64_t* l_off, const int64_t* x_off, double* X);
   int prepare_rhs(const double* fu);
