@@ -1565,8 +1565,9 @@ __global__ void __launch_bounds__(512) k_block_colgemv(int32_t n_mat, const int3
 // adds a root's slots in order.  kR rows at a time share one block sum (a warp
 // reduce-scatter, then every warp adds the 16 warps' values in the same order:
 // one barrier).  The rows of the next steps are on their way into a ring in
-// shared memory meanwhile, as bulk copies by one thread: 160 to 200 KB in flight
-// an SM without a register or an issue slot of the threads that compute.  A row
+// shared memory meanwhile, as bulk copies by one thread: a ring of two to five
+// steps (164 to 197 KB of the longest rows of each kK)
+// without a register or an issue slot of the threads that compute.  A row
 // is copied from the 16-byte boundary at or before its start.  The waits are
 // bounded: one that runs out sets kErrWait, and the product becomes NaN.
 // Split: by entries + kTriRowCost a row.  With the entries alone the CTAs of the
@@ -1583,7 +1584,7 @@ __global__ void __launch_bounds__(512) k_block_colgemv(int32_t n_mat, const int3
 // dots 1.67e-16 to 2.04e-16; without the carried roundings of add_carried it was
 // 1.9e-16 to 3.3e-16.  S w needs none: the tile pass adds a quarter of a row in
 // one chain, here it is 128 sums of kR.
-constexpr int kTriT = 512, kTriMaxK = 8, kTriRing = 24600, kTriStages = 8;
+constexpr int kTriT = 512, kTriMaxK = 8, kTriRing = 24624, kTriStages = 8;
 constexpr int32_t kTriMaxN = kTriT * kTriMaxK;
 constexpr int64_t kTriRowCost = 3072;  // what a row costs beside its entries, in entries
 constexpr int64_t kTriMinRow = 384, kTriMinEntries = 2000000;
@@ -1609,6 +1610,8 @@ __device__ __forceinline__ bool tri_rows(const T* __restrict__ M, int64_t off, i
                                          double2* __restrict__ out) {
   static_assert(kR <= 8 && kTriT == 512, "a lane adds kR / 2 of the 16 warps' values");
   constexpr int V = 16 / sizeof(T);
+  static_assert(kTriRing * sizeof(double) >= 2 * kR * ((kTriT * kK + 2 * V - 2) / V * V) * sizeof(T),
+                "a step's rows on their way while those of the step before are used");
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
   const int cap = (rb + 2 * V - 2) / V * V;  // a row from the boundary before it, whole vectors
   const int depth = min(kTriStages, static_cast<int>(kTriRing * sizeof(double) / (kR * cap * sizeof(T))));
