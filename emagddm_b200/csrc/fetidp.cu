@@ -1565,11 +1565,11 @@ __global__ void __launch_bounds__(512) k_block_colgemv(int32_t n_mat, const int3
 // adds a root's slots in order.  kR rows at a time share one block sum (a warp
 // reduce-scatter, then every warp adds the 16 warps' values in the same order:
 // one barrier).  The rows of the next steps are on their way into a ring in
-// shared memory meanwhile, as bulk copies by one thread: a ring of two to five
-// steps (164 to 197 KB of the longest rows of each kK)
-// without a register or an issue slot of the threads that compute.  A row
-// is copied from the 16-byte boundary at or before its start.  The waits are
-// bounded: one that runs out sets kErrWait, and the product becomes NaN.
+// shared memory meanwhile, as bulk copies by one thread, without a register or an
+// issue slot of the threads that compute: two to five steps of the longest rows of
+// a kK, 164 to 197 KB an SM.  A row is copied from the 16-byte boundary at or
+// before its start.  The waits are bounded: one that runs out sets kErrWait, and
+// the product becomes NaN.
 // Split: by entries + kTriRowCost a row.  With the entries alone the CTAs of the
 // short rows take three times as long as the others (64 roots of 1,500 to 3,100
 // unknowns, 1.39 GB: 554 us at 0, 333 at 512, 311 at 1024, 289 at 2048 to 4096).
