@@ -1015,6 +1015,10 @@ def run_learned(args, rank, world, local_rank):
 
 def run_reference(args):
     from oracle import oracle as O
+    from oracle import refbridge as R
+    if not R.available():
+        return {"impl": "reference", "unavailable": "the reference's solver library (oracle/_ref/libemg_ref.so, built "
+                                                    "from the reference's sources) is not there"}
     m = workload(args.n)
     dof = O.dof_build(m.tets, m.dirichlet, gauge=O.GAUGE_REF)
     l2g = dof["l2g"]
