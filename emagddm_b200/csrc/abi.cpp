@@ -825,8 +825,8 @@ int32_t emg_tune_report(char* buf, int32_t cap) {
 
 int emg_test_set_barrier_spins(int32_t spins) {
   return guarded([&]() -> int {
-    const int rc = emg::set_barrier_spins(spins);
-    return rc ? rc : emg::set_front_polls(spins);
+    emg::set_front_polls(spins);
+    return emg::set_barrier_spins(spins);
   });
 }
 

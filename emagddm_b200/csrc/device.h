@@ -108,7 +108,7 @@ int bicgstab_solve(DevCsr& A, const double* b, double* x, const emg_krylov_confi
 int csr_history(DevCsr& A, double* out, int32_t cap);
 int cg_kernel_times(DevCsr& A, int32_t iterations, cudaStream_t st, double* ms);
 int set_barrier_spins(int32_t spins);
-int set_front_polls(int32_t polls);  // fetidp.cu
+void set_front_polls(int32_t polls);  // fetidp.cu
 void set_resident(bool on);
 void free_workspace(KrylovWorkspace* ws);
 void free_batch(BatchPlan* p);

@@ -19,6 +19,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdlib>
 #include <string>
@@ -1044,9 +1045,12 @@ __global__ void __launch_bounds__(kPivMax) k_front_bwd_piv(FrontsDev F, int32_t 
 // one pass takes 7.0 ms there and 1.1 ms here.
 constexpr int kRB = kNB;  // rows of a block
 constexpr int32_t kWaitPolls = 1 << 22;
-// Polls a waiting block of the front solves and of the root products makes before
-// it gives up; kWaitPolls unless a test lowers it (emg_test_set_barrier_spins).
-__device__ int32_t g_wait_polls = kWaitPolls;
+// Polls that a waiting block of the front solves makes before it gives up;
+// kWaitPolls unless a test lowers it (emg_test_set_barrier_spins; 0 also makes the
+// root products give up, whose limit is tma::kSpinLimit).  An argument of the
+// kernels, loaded by them it cost a right-hand side on the 24^3 direct factor 28 us
+// of 1,085; as the bound of the root products' wait it cost 64^3 0.7 ms of 54.
+std::atomic<int32_t> g_front_polls{kWaitPolls};
 
 __device__ __forceinline__ int32_t ld_acquire(const int32_t* p) {
   int32_t v;
@@ -1066,14 +1070,14 @@ __device__ __forceinline__ int32_t wait_progress(const int32_t* p, int32_t want,
   return -1;
 }
 
-__global__ void __launch_bounds__(256) k_front_fwd_rows(FrontsDev F, int32_t f0, int32_t nf, RhsDev R,
+__global__ void __launch_bounds__(256, 3) k_front_fwd_rows(FrontsDev F, int32_t f0, int32_t nf, RhsDev R,
                                                         const double* __restrict__ fac, int32_t* __restrict__ ticket,
-                                                        int32_t* __restrict__ prog, int32_t* __restrict__ err) {
+                                                        int32_t* __restrict__ prog, int32_t* __restrict__ err,
+                                                        int32_t polls) {
   __shared__ int32_t tk;
   __shared__ double xs[kRB], vs[kRB], ys[2][kRB], part[4][kRB];
   __shared__ double X[kRB][kRB + 1];  // X[r][c] = (L_II^-1)(r, c)
   const int t = threadIdx.x, r = t & (kRB - 1), g = t >> 6;
-  const int32_t polls = g_wait_polls;
   if (t == 0) tk = atomicAdd(ticket, 1);
   __syncthreads();
   const int32_t b = tk / nf, k = f0 + (tk - b * nf);
@@ -1161,13 +1165,13 @@ __global__ void __launch_bounds__(256) k_front_fwd_rows(FrontsDev F, int32_t f0,
   if (t == 0) st_release(prog + k, b + 1);
 }
 
-__global__ void __launch_bounds__(256) k_front_bwd_rows(FrontsDev F, int32_t f0, int32_t nf, RhsDev R,
+__global__ void __launch_bounds__(256, 2) k_front_bwd_rows(FrontsDev F, int32_t f0, int32_t nf, RhsDev R,
                                                         const double* __restrict__ fac, int32_t* __restrict__ ticket,
-                                                        int32_t* __restrict__ prog, int32_t* __restrict__ err) {
+                                                        int32_t* __restrict__ prog, int32_t* __restrict__ err,
+                                                        int32_t polls) {
   __shared__ int32_t tk;
   __shared__ double dots[kRB], vs[kRB], part[4][kRB];
   const int t = threadIdx.x, lane = t & 31, w = t >> 5, r = t & (kRB - 1), g = t >> 6;
-  const int32_t polls = g_wait_polls;
   if (t == 0) tk = atomicAdd(ticket, 1);
   __syncthreads();
   const int32_t q = tk / nf, k = f0 + (tk - q * nf);
@@ -1631,7 +1635,7 @@ __device__ __forceinline__ bool tri_rows(const T* __restrict__ M, int64_t off, i
     for (int i = 0; i < min(depth, steps); ++i) fetch(i, i);
   double acc[kK] = {};
   for (int i = 0, stage = 0, buf = 0; i < steps; ++i, buf ^= 1) {
-    const bool ok = tma::mbar_wait(sm.full + stage, (phase >> stage) & 1u, polls);
+    const bool ok = tma::mbar_wait(sm.full + stage, (phase >> stage) & 1u) && polls > 0;
     const int32_t r = ra + i * kR;
     double v[kR][kK], s[kR];
 #pragma unroll
@@ -1714,14 +1718,13 @@ __global__ void __launch_bounds__(kTriT, 1) k_tri_apply(const TriSeg* __restrict
                                                        const int64_t* __restrict__ m_off, const T* __restrict__ M,
                                                        const int64_t* __restrict__ v_off,
                                                        const double* __restrict__ w, double2* __restrict__ slots,
-                                                       int32_t* __restrict__ err) {
+                                                       int32_t* __restrict__ err, uint32_t polls) {
   extern __shared__ __align__(128) double smd[];
   const TriSmem sm{smd, smd + kTriRing, smd + kTriRing + kTriMaxN,
                    reinterpret_cast<uint64_t*>(smd + kTriRing + kTriMaxN + kTriRed)};
   if (threadIdx.x < kTriStages) tma::mbar_init(sm.full + threadIdx.x, 1);
   tma::fence_mbar_init();
   const uint64_t pol = evict_first_policy();
-  const uint32_t polls = static_cast<uint32_t>(g_wait_polls);
   uint32_t phase = 0;
   bool ok = true;
   for (int32_t g = cta_seg[blockIdx.x]; g < cta_seg[blockIdx.x + 1]; ++g) {
@@ -2705,10 +2708,9 @@ int FetiDP::setup_device() {
   return EMG_SUCCESS;
 }
 
-int set_front_polls(int32_t polls) {
+void set_front_polls(int32_t polls) {
   const int32_t v = polls < 0 ? kWaitPolls : polls;
-  EMG_CK(cudaMemcpyToSymbol(g_wait_polls, &v, sizeof(v)));
-  return EMG_SUCCESS;
+  g_front_polls = v;
 }
 
 int FetiDP::check_err(const char* where) {
@@ -2916,7 +2918,7 @@ int FetiDP::solve_fronts(const RhsDev& R, int32_t ncol) {
     if (ncol == 1) {
       if (lvl_max_blk[h] > 0)
         k_front_fwd_rows<<<static_cast<unsigned>(lvl_max_blk[h]) * static_cast<unsigned>(nf), 256, 0, st>>>(
-            fd, f0, nf, R, fac_d, tick + h, prog_d, err_d);
+            fd, f0, nf, R, fac_d, tick + h, prog_d, err_d, g_front_polls);
       continue;
     }
     k_front_fwd_piv<<<dim3(nc, static_cast<unsigned>(nf)), piv_threads, 0, st>>>(fd, f0, R, d_nI, d_nD, fac_d);
@@ -2954,7 +2956,7 @@ int FetiDP::solve_fronts(const RhsDev& R, int32_t ncol) {
     if (ncol == 1) {
       const int32_t nb = (lvl_max_np[h] + kRB - 1) / kRB;
       k_front_bwd_rows<<<static_cast<unsigned>(nb) * static_cast<unsigned>(nf), 256, 0, st>>>(
-          fd, f0, nf, R, fac_d, tick + nlev + h, prog_d + F, err_d);
+          fd, f0, nf, R, fac_d, tick + nlev + h, prog_d + F, err_d, g_front_polls);
       continue;
     }
     if (lvl_max_nu[h] > 0)
@@ -2979,7 +2981,8 @@ void FetiDP::coarse_apply_t(const RhsDev& R, const double* w, const double* add,
 template <bool kInverse, class T>
 void FetiDP::tri_apply(const T* M, const double* w, double* y) {
   k_tri_apply<kInverse, T><<<tri_ctas, kTriT, kTriSmem, st>>>(d_tri_seg, d_tri_cta, d_rdim, d_roff, M, d_rvoff, w,
-                                                             tri_slots_d, err_d);
+                                                             tri_slots_d, err_d,
+                                                             static_cast<uint32_t>(g_front_polls.load()));
   k_tri_sum<<<dim3(blocks_for(max_nD, 256), static_cast<unsigned>(n_roots)), 256, 0, st>>>(
       d_tri_seg, d_tri_root, d_rdim, d_rvoff, tri_slots_d, y);
 }
@@ -3406,6 +3409,11 @@ cudaGraphExec_t FetiDP::lambda_loop_graph() {
     return e && e[0] == '0';
   }();
   if (off || graph_failed) return nullptr;
+  if (lam_polls != g_front_polls) {  // the captured loops hold another poll limit
+    for (cudaGraphExec_t& g : lam_exec)
+      if (g) { cudaGraphExecDestroy(g); g = nullptr; }
+    lam_polls = g_front_polls;
+  }
   if (lam_exec[precond]) return lam_exec[precond];
   if (!cap_st && cudaStreamCreateWithFlags(&cap_st, cudaStreamNonBlocking) != cudaSuccess) {
     cudaGetLastError();

@@ -149,6 +149,7 @@ struct FetiDP {
                               // level the block tickets (forward, backward)
   // device-side multiplier loop: one while-loop graph per preconditioner 0..3
   cudaGraphExec_t lam_exec[4] = {nullptr, nullptr, nullptr, nullptr};
+  int32_t lam_polls = 0;  // poll limit in them
   cudaStream_t cap_st = nullptr;
   // second stream of the captured factorization: the deluxe face set-up
   // (which needs only the assembled S_DD blocks) beside the root inverse

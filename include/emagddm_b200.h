@@ -487,8 +487,9 @@ int32_t emg_tune_report(char* buf, int32_t cap);
 /* Test hook (no counterpart in the reference): polls that a waiting block
  * makes before it gives up, at the grid barrier of the fused CG update and of
  * the resident solves (default 2^21, about 0.2 s or more) and in the front
- * solves and root products of FETI-DP and the direct solver (2^22); a negative
- * value restores the defaults.  On the current device.  A block that gives up
+ * solves of FETI-DP and the direct solver (2^22; 0 also makes the root products
+ * of FETI-DP give up); a negative value restores the defaults.  On the current
+ * device.  A block that gives up
  * ends the solve with EMG_ERR_TIMEOUT instead of waiting on; tests lower the
  * limit to make these waits run out. */
 int emg_test_set_barrier_spins(int32_t spins);
