@@ -584,9 +584,9 @@ __device__ __forceinline__ bool reduce_partials(const double (&vals)[kVals], dou
 }
 
 // ------------------------------------------------------------ SELL build ----
-// Warp per slice: column index (permuted), own column (for products in the
-// matrix's own numbering) and CSR source of every slot; rows at or past n are
-// all padding.
+// Warp per slice: column index (permuted), CSR source and, for products in the
+// matrix's own numbering (ocol not null), own column of every slot; rows at or
+// past n are all padding.
 __global__ void k_sell_fill(int64_t n, int64_t nslices, const int64_t* __restrict__ sp,
                             const int32_t* __restrict__ perm, const int32_t* __restrict__ iperm,
                             const int32_t* __restrict__ rp, const int32_t* __restrict__ ccol,
@@ -607,7 +607,7 @@ __global__ void k_sell_fill(int64_t n, int64_t nslices, const int64_t* __restric
     }
     for (int j = 0; j < len; ++j) {
       const int64_t k = b0 + static_cast<int64_t>(kSliceRows) * j + lane;
-      ocol[k] = j < rl ? ccol[a + j] : 0;
+      if (ocol) ocol[k] = j < rl ? ccol[a + j] : 0;
       if (j < rl) {
         col[k] = iperm[ccol[a + j]];
         src[k] = a + j;
@@ -730,16 +730,26 @@ __global__ void k_scatter(int64_t n, const int32_t* __restrict__ perm, const dou
   for (int64_t i = gtid(); i < n; i += gstride()) out[perm[i]] = in[i];
 }
 
+__global__ void k_sell_own_columns(int64_t slots, const int32_t* __restrict__ src, const int32_t* __restrict__ ccol,
+                                   int32_t* __restrict__ ocol) {
+  for (int64_t i = gtid(); i < slots; i += gstride()) ocol[i] = src[i] >= 0 ? ccol[src[i]] : 0;
+}
+
+__global__ void k_gather(int64_t n, const int32_t* __restrict__ perm, const double* __restrict__ in,
+                         double* __restrict__ out) {
+  for (int64_t i = gtid(); i < n; i += gstride()) out[i] = in[perm[i]];
+}
+
 // y = A x in the matrix's own numbering: the slots' own columns and rows
 // written through the permutation, so a product is one launch.  (Gathering x
 // into the solvers' numbering and scattering y out of it took three launches
 // and a memset: 13.4 us for 990 rows and 65 us for the 64^3 matrix.)  Padding
 // and masked entries multiply x[0] by 0, so a row that is no number is formed
 // again from its own entries alone (reading no x for padding in the first place
-// cost every product 2 us of 44 at 64^3).
+// cost every product 2 us of 44 at 64^3).  A.col, x: the own columns, or the
+// solvers' with x in their numbering.
 __global__ void __launch_bounds__(kThreads) k_product(Sell A, const int32_t* __restrict__ perm,
                                                       const double* __restrict__ x, double* __restrict__ y) {
-  A.col = A.ocol;
   sell_rows(A, x, [&](int64_t row, double s) {
     if (!isfinite(s)) {
       int64_t base;
@@ -750,7 +760,7 @@ __global__ void __launch_bounds__(kThreads) k_product(Sell A, const int32_t* __r
 #pragma unroll 1  // unrolled it takes 74 registers, a block less an SM
       for (int j = 0; j < len; ++j) {
         const int64_t k = base + static_cast<int64_t>(kSliceRows) * j;
-        if (A.src[k] >= 0) s += A.val[k] * x[A.ocol[k]];
+        if (A.src[k] >= 0) s += A.val[k] * x[A.col[k]];
       }
     }
     y[perm[row]] = s;
@@ -1337,7 +1347,7 @@ int grid_size() {
 
 // Host: permutation sorting rows by length inside windows (stable), slice
 // offsets; device: slots.
-int build_sell(DevCsr& A, cudaStream_t st) {
+int build_sell(DevCsr& A, bool own_columns, cudaStream_t st) {
   if (!A.sell) A.sell = new Sell();
   Sell& S = *A.sell;
   const int64_t n = A.n;
@@ -1372,7 +1382,7 @@ int build_sell(DevCsr& A, cudaStream_t st) {
   const size_t ns = static_cast<size_t>(std::max<int64_t>(S.slots, 1));
   EMG_CK(cudaMallocAsync(&iperm, sizeof(int32_t) * n, st));
   EMG_CK(cudaMallocAsync(&S.src, sizeof(int32_t) * ns, st));
-  EMG_CK(cudaMallocAsync(&S.ocol, sizeof(int32_t) * ns, st));
+  if (own_columns) EMG_CK(cudaMallocAsync(&S.ocol, sizeof(int32_t) * ns, st));
   EMG_CK(cudaMallocAsync(&S.col, sizeof(int32_t) * ns, st));
   EMG_CK(cudaMallocAsync(&S.val, sizeof(double) * ns, st));
   k_invert_perm<<<g, kThreads, 0, st>>>(n, S.perm, iperm);
@@ -1440,10 +1450,11 @@ int build_sell(DevCsr& A, cudaStream_t st) {
 
 void tune_sell_grid(DevCsr& A, cudaStream_t st);
 
-int ensure_sell(DevCsr& A, cudaStream_t st) {
+// own_columns: products in the matrix's own numbering (csr_spmv) will be asked for
+int ensure_sell(DevCsr& A, cudaStream_t st, bool own_columns = false) {
   bool fresh = false;
   if (!A.sell) {
-    int rc = build_sell(A, st);
+    int rc = build_sell(A, own_columns, st);
     if (rc) return rc;
     fresh = true;
   }
@@ -1817,9 +1828,11 @@ void tune_sell_grid(DevCsr& A, cudaStream_t st) {
   for (int d = 1; d <= 2; ++d)
     if (r - d * sms >= sms) cand.push_back(r - d * sms);
   const std::string key = "n" + std::to_string(A.n) + "slots" + std::to_string(S.slots);
-  cudaMemsetAsync(A.ws->p, 0, sizeof(double) * A.n, st);  // no rows that are no number
+  bool cleared = false;
   S.grid = tune::pick("sell.spmv_grid", key, cand, [&](int v, cudaStream_t s) {
-    k_product<<<v, kThreads, 0, s>>>(S, S.perm, A.ws->p, A.ws->q);
+    if (!cleared) cudaMemsetAsync(A.ws->p, 0, sizeof(double) * A.n, s);  // no rows that are no number
+    cleared = true;
+    k_product<<<v, kThreads, 0, s>>>(S, S.perm, A.ws->p, A.ws->q);  // any columns do
   }, st);
   cudaGetLastError();
 }
@@ -1983,17 +1996,32 @@ int csr_spmv(DevCsr& A, const double* x, double* y, cudaStream_t st) {
   if (!x || !y) { set_error("null vector"); return EMG_INVALID_INPUT; }
   int rc = ensure_ws(A, false, 1, st);
   if (rc) return rc;
-  rc = ensure_sell(A, st);
+  rc = ensure_sell(A, st, true);
   if (rc) return rc;
-  const Sell& S = *A.sell;
+  Sell& S = *A.sell;
+  if (!S.ocol) {  // built by a solver, which does without (64^3 solve: 0.6 ms with them)
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    EMG_CK(cudaStreamIsCapturing(st, &cs));
+    if (cs == cudaStreamCaptureStatusNone) {  // an allocation would belong to the captured graph
+      EMG_CK(cudaMallocAsync(&S.ocol, sizeof(int32_t) * std::max<int64_t>(S.slots, 1), st));
+      k_sell_own_columns<<<grid_size(), kThreads, 0, st>>>(S.slots, S.src, A.col, S.ocol);
+    }
+  }
   const int64_t warps = std::max<int64_t>(S.nslices, 1);
   const int grid = static_cast<int>(std::min<int64_t>(sell_grid<k_product>(S, grid_size()),
                                                       (warps + kThreads / 32 - 1) / (kThreads / 32)));
+  Sell P = S;
+  if (S.ocol) {
+    P.col = S.ocol;
+  } else {
+    k_gather<<<grid_size(), kThreads, 0, st>>>(A.n, S.perm, x, A.ws->p);
+    x = A.ws->p;
+  }
   if (x < y + A.n && y < x + A.n) {  // the operands overlap: rows are written while others still read x
     EMG_CK(cudaMemcpyAsync(A.ws->p, x, sizeof(double) * A.n, cudaMemcpyDeviceToDevice, st));
     x = A.ws->p;
   }
-  k_product<<<grid, kThreads, 0, st>>>(S, S.perm, x, y);
+  k_product<<<grid, kThreads, 0, st>>>(P, S.perm, x, y);
   EMG_CK(cudaGetLastError());
   return EMG_SUCCESS;
 }

@@ -283,7 +283,7 @@ __global__ void __launch_bounds__(T, 1) k_cg_resident(ResidentArgs P) {
 #pragma unroll
   for (int q = 0; q < NR; ++q)
     if (R.live[q]) P.x[P.A.perm[R.row[q]]] = x[q];
-  if (threadIdx.x == 0 && sh_bad) atomicOr(&P.st->copy_err, 1);
+  if (threadIdx.x == 0 && status == EMG_ERR_TIMEOUT) atomicOr(&P.st->copy_err, 1);
   if (writer) {
     P.st->status = status;
     P.st->iter = it;
@@ -393,7 +393,7 @@ __global__ void __launch_bounds__(T, 1) k_bi_resident(ResidentArgs P) {
 #pragma unroll
   for (int q = 0; q < NR; ++q)
     if (R.live[q]) P.x[P.A.perm[R.row[q]]] = x[q];
-  if (threadIdx.x == 0 && sh_bad) atomicOr(&P.st->copy_err, 1);
+  if (threadIdx.x == 0 && status == EMG_ERR_TIMEOUT) atomicOr(&P.st->copy_err, 1);
   if (writer) {
     P.st->status = status;
     P.st->iter = it;
