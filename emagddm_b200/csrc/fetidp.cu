@@ -392,9 +392,9 @@ constexpr int kGK = 16;  // k-chunk of the tile GEMM
 // the issue of shared-memory loads beside the tensor work, hence the 16-row
 // fragments (m8n8k4 with a warp on 8 rows x 64 columns took 9 loads for 8
 // products of a quarter the size) and, for larger blocks, M = 128, which also
-// halves the reads of B from L2.  The FP64 pipe is 75 % busy on the largest
-// levels (37 TFLOP/s is its rate; three buffers instead of two changed
-// nothing); the pivot-column updates of the 33^3 direct factor went from 7.6 to
+// halves the reads of B from L2.  The tensor pipe is active 71 to 78 % of the
+// cycles in the largest launches of the 33^3 direct factor (three buffers
+// instead of two changed nothing); its pivot-column updates went from 7.6 to
 // 6.9 ms, those of the 64^3 FETI-DP factor from 28.1 to 27.0.
 constexpr int kMmaThreads = 256;
 constexpr int kMmaPad = kTile + 4;

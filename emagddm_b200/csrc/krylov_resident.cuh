@@ -4,7 +4,7 @@
 // A solve of a few ten thousand unknowns is bound by latency, not by bytes:
 // the loop graph runs two (CG) or five (BiCGSTAB) dependent launches an
 // iteration, 17 us for the 22,320 rows of the 16^3 problem whose 3.4 MB matrix
-// the SMs could read in one (7 us here; BiCGSTAB on 67,712 rows of 33^3
+// the SMs could read in one (8 us here; BiCGSTAB on 67,712 rows of 33^3
 // hexahedra 33 -> 14 us).  Here one block per SM owns a contiguous run of
 // slices for the whole solve: its part of the matrix is staged in shared
 // memory once (as many slices as fit; the rest is read through L2), a lane
