@@ -744,7 +744,7 @@ __global__ void k_gather(int64_t n, const int32_t* __restrict__ perm, const doub
 // written through the permutation, so a product is one launch.  (Gathering x
 // into the solvers' numbering and scattering y out of it took three launches
 // and a memset: 13.4 us for 990 rows and 65 us for the 64^3 matrix.)  Padding
-// and masked entries multiply x[0] by 0, so a row that is no number is formed
+// and masked entries multiply an x by 0, so a row that is no number is formed
 // again from its own entries alone (reading no x for padding in the first place
 // cost every product 2 us of 44 at 64^3).  A.col, x: the own columns, or the
 // solvers' with x in their numbering.
@@ -1999,7 +1999,7 @@ int csr_spmv(DevCsr& A, const double* x, double* y, cudaStream_t st) {
   rc = ensure_sell(A, st, true);
   if (rc) return rc;
   Sell& S = *A.sell;
-  if (!S.ocol) {  // built by a solver, which does without (64^3 solve: 0.6 ms with them)
+  if (!S.ocol) {  // built by a solver, which does without
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     EMG_CK(cudaStreamIsCapturing(st, &cs));
     if (cs == cudaStreamCaptureStatusNone) {  // an allocation would belong to the captured graph

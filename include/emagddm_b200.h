@@ -307,7 +307,9 @@ int emg_fetidp_learned_train(emg_fetidp fd, int32_t batch, const double* r_d, co
 /* FP32 master parameters (host array of *n floats): load != 0 copies in. */
 int emg_fetidp_learned_params(emg_fetidp fd, float* params, int64_t* n, int32_t load);
 /* Multiplier space, device vectors of n_lambda (emg_fetidp_info[3]):
- * op 0 F, 1 deluxe Dirichlet M_D, 2 learned correction L, 3 M_D + L. */
+ * op 0 F, 1 deluxe Dirichlet M_D, 2 learned correction L, 3 M_D + L.  Returns
+ * when out_d is ready, EMG_ERR_TIMEOUT where a bounded wait ran out; while the
+ * solver's stream is captured it only enqueues, and such a wait shows as NaN. */
 int emg_fetidp_apply(emg_fetidp fd, int32_t op, const double* in_d, double* out_d);
 /* Right-hand side d - G S_cc^-1 g_c of the multiplier system for a global b
  * (device, n_dofs; NULL = the assembled F) into rhs_d (device, n_lambda). */
