@@ -746,11 +746,13 @@ __global__ void k_gather(int64_t n, const int32_t* __restrict__ perm, const doub
 // and a memset: 13.4 us for 990 rows and 65 us for the 64^3 matrix.)  Padding
 // and masked entries multiply an x by 0, so a row that is no number is formed
 // again from its own entries alone (reading no x for padding in the first place
-// cost every product 2 us of 44 at 64^3).  A.col, x: the own columns, or the
+// cost every product 2 us of 44 at 64^3).  col, x: the own columns, or the
 // solvers' with x in their numbering.
-__global__ void __launch_bounds__(kThreads) k_product(Sell A, const int32_t* __restrict__ perm,
+__global__ void __launch_bounds__(kThreads) k_product(Sell A, int32_t* col, const int32_t* __restrict__ perm,
                                                       const double* __restrict__ x, double* __restrict__ y) {
+  A.col = col;
   sell_rows(A, x, [&](int64_t row, double s) {
+    const int32_t at = perm[row];  // on its way beside the last products
     if (!isfinite(s)) {
       int64_t base;
       int len;
@@ -763,7 +765,7 @@ __global__ void __launch_bounds__(kThreads) k_product(Sell A, const int32_t* __r
         if (A.src[k] >= 0) s += A.val[k] * x[A.col[k]];
       }
     }
-    y[perm[row]] = s;
+    y[at] = s;
   });
 }
 
@@ -1832,7 +1834,7 @@ void tune_sell_grid(DevCsr& A, cudaStream_t st) {
   S.grid = tune::pick("sell.spmv_grid", key, cand, [&](int v, cudaStream_t s) {
     if (!cleared) cudaMemsetAsync(A.ws->p, 0, sizeof(double) * A.n, s);  // no rows that are no number
     cleared = true;
-    k_product<<<v, kThreads, 0, s>>>(S, S.perm, A.ws->p, A.ws->q);  // any columns do
+    k_product<<<v, kThreads, 0, s>>>(S, S.col, S.perm, A.ws->p, A.ws->q);
   }, st);
   cudaGetLastError();
 }
@@ -2010,10 +2012,9 @@ int csr_spmv(DevCsr& A, const double* x, double* y, cudaStream_t st) {
   const int64_t warps = std::max<int64_t>(S.nslices, 1);
   const int grid = static_cast<int>(std::min<int64_t>(sell_grid<k_product>(S, grid_size()),
                                                       (warps + kThreads / 32 - 1) / (kThreads / 32)));
-  Sell P = S;
-  if (S.ocol) {
-    P.col = S.ocol;
-  } else {
+  // (an argument: a second copy of S to hold it costs a call 0.4 us of 7.4)
+  int32_t* col = S.ocol ? S.ocol : S.col;
+  if (!S.ocol) {
     k_gather<<<grid_size(), kThreads, 0, st>>>(A.n, S.perm, x, A.ws->p);
     x = A.ws->p;
   }
@@ -2021,7 +2022,7 @@ int csr_spmv(DevCsr& A, const double* x, double* y, cudaStream_t st) {
     EMG_CK(cudaMemcpyAsync(A.ws->p, x, sizeof(double) * A.n, cudaMemcpyDeviceToDevice, st));
     x = A.ws->p;
   }
-  k_product<<<grid, kThreads, 0, st>>>(P, S.perm, x, y);
+  k_product<<<grid, kThreads, 0, st>>>(S, col, S.perm, x, y);
   EMG_CK(cudaGetLastError());
   return EMG_SUCCESS;
 }
