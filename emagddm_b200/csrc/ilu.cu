@@ -843,19 +843,25 @@ cudaGraphExec_t ilu_loop_graph(DevCsr& A, IluState& s, bool bicg) {
   return exec;
 }
 
+int ilu_setup(DevCsr& A, IluState& s, cudaStream_t st) {
+  s.n = A.n;
+  s.nnz = A.nnz;
+  int rc = ilu_symbolic(A, s, st);
+  if (rc || s.failed) return rc;
+  for (double** v : {&s.x, &s.r, &s.z, &s.p, &s.q, &s.y, &s.rh, &s.v, &s.s, &s.t})
+    if ((rc = ilu_alloc(s, v, A.n))) return rc;
+  if ((rc = ilu_alloc(s, &s.part, 2 * kIlGrid)) || (rc = ilu_alloc(s, &s.st, 1))) return rc;
+  return EMG_SUCCESS;
+}
+
 int ilu_prepare(DevCsr& A, cudaStream_t st) {
   if (!A.ilu) {
     A.ilu = new IluState();
-    IluState& s = *A.ilu;
-    s.n = A.n;
-    s.nnz = A.nnz;
-    int rc = ilu_symbolic(A, s, st);
-    if (rc) return rc;
-    if (!s.failed) {
-      const int64_t n = A.n;
-      for (double** v : {&s.x, &s.r, &s.z, &s.p, &s.q, &s.y, &s.rh, &s.v, &s.s, &s.t})
-        if ((rc = ilu_alloc(s, v, n))) return rc;
-      if ((rc = ilu_alloc(s, &s.part, 2 * kIlGrid)) || (rc = ilu_alloc(s, &s.st, 1))) return rc;
+    if (const int rc = ilu_setup(A, *A.ilu, st)) {  // nothing half prepared stays
+      free_ilu(A.ilu);
+      A.ilu = nullptr;
+      cudaGetLastError();
+      return rc;
     }
   }
   IluState& s = *A.ilu;

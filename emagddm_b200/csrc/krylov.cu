@@ -1451,12 +1451,26 @@ int build_sell(DevCsr& A, bool own_columns, cudaStream_t st) {
 }
 
 void tune_sell_grid(DevCsr& A, cudaStream_t st);
+void free_sell(Sell* s);
+
+int refuse_capture(cudaStream_t st) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  EMG_CK(cudaStreamIsCapturing(st, &cs));
+  if (cs == cudaStreamCaptureStatusNone) return EMG_SUCCESS;
+  set_error("the first use of a matrix allocates and cannot be captured");
+  return EMG_ERR_CUDA;
+}
 
 // own_columns: products in the matrix's own numbering (csr_spmv) will be asked for
 int ensure_sell(DevCsr& A, cudaStream_t st, bool own_columns = false) {
   bool fresh = false;
   if (!A.sell) {
-    int rc = build_sell(A, own_columns, st);
+    int rc = refuse_capture(st);
+    if (!rc && (rc = build_sell(A, own_columns, st))) {
+      free_sell(A.sell);
+      A.sell = nullptr;
+      cudaGetLastError();
+    }
     if (rc) return rc;
     fresh = true;
   }
@@ -1716,7 +1730,7 @@ bool launch_resident(DevCsr& A, const double* b, double* x, int32_t precond, boo
   return e == cudaSuccess;
 }
 
-int ensure_ws(DevCsr& A, bool bicg, int32_t max_iter, cudaStream_t st) {
+int prepare_ws(DevCsr& A, bool bicg, int32_t max_iter, cudaStream_t st) {
   if (!A.ws) {
     A.ws = new KrylovWorkspace();
     KrylovWorkspace& w = *A.ws;
@@ -1754,6 +1768,20 @@ int ensure_ws(DevCsr& A, bool bicg, int32_t max_iter, cudaStream_t st) {
       if (*g) { cudaGraphExecDestroy(*g); *g = nullptr; }
   }
   return EMG_SUCCESS;
+}
+
+// What is prepared is prepared whole: under capture, where allocations would
+// belong to the graph, nothing is, and a preparation that fails leaves nothing.
+int ensure_ws(DevCsr& A, bool bicg, int32_t max_iter, cudaStream_t st) {
+  if (A.ws && max_iter <= A.ws->hist_cap && (!bicg || A.ws->rh)) return EMG_SUCCESS;
+  if (const int rc = refuse_capture(st)) return rc;
+  const int rc = prepare_ws(A, bicg, max_iter, st);
+  if (rc) {
+    free_workspace(A.ws);
+    A.ws = nullptr;
+    cudaGetLastError();
+  }
+  return rc;
 }
 
 void launch_iterations(DevCsr& A, bool bicg, int count);

@@ -56,3 +56,31 @@ def test_captured_product_after_a_solve():
         product(xd, yd)
         torch.cuda.synchronize()
         assert np.abs(yd.cpu().numpy() - want(x)).max() <= 1e-13 * 100
+
+
+def test_first_use_under_capture_is_refused_and_leaves_nothing():
+    """A matrix that nothing has used yet allocates: refused while the stream is
+    captured, without ending the capture, and good afterwards."""
+    import torch
+    n = 1000
+    i = np.arange(n, dtype=np.int32)
+    A = HostCsr(np.arange(n + 1, dtype=np.int32), i, 2.0 + i)
+    x = torch.ones(n, dtype=torch.float64, device="cuda")
+    y = torch.zeros_like(x)
+    z = torch.zeros_like(x)
+    rc = []
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+        rc.append(lib().emg_spmv(A.h, C.c_void_p(x.data_ptr()), C.c_void_p(y.data_ptr()), stream))
+        z.add_(1.0)
+    assert rc[0] == _abi.EMG_ERR_CUDA and b"captured" in lib().emg_last_error()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert (z == 1.0).all() and (y == 0.0).all()
+    del graph
+    _abi.check(lib().emg_spmv(A.h, C.c_void_p(x.data_ptr()), C.c_void_p(y.data_ptr()), None), "emg_spmv")
+    torch.cuda.synchronize()
+    assert np.array_equal(y.cpu().numpy(), 2.0 + i)
+    b, out = solve(A.h, np.ones(n), "cg", tol=1e-10, precond=1)
+    assert out.status == 0
